@@ -270,70 +270,113 @@ sparse_scan_kernel(const int32_t* __restrict__ bin_count, int32_t* __restrict__ 
 
 // ------------------------------------------------------------------------------------------
 // merge: out[t, h] = sum_s w_s O_s / sum_s w_s over the selections of (t, kv head), w_s = exp(lse_s - max)
-// Half a warp per (token, head) row, lane l of the half owns columns 8l..8l+7.  Rows are walked in
-// output order, which is also the order of the partial buffer: the kbn x G partial rows of a
-// (token, kv head) are one contiguous block, so the pass streams.  All loads of a row are issued
-// before any is used.
+// HBM-bound (kbn * 260 bytes in, 256 out per row).  Half a warp per (token, head) row, a lane owns one 16-byte
+// piece of it in every slot.  Rows are walked in output order, which is also the order of the partial buffer:
+// the kbn x G partial rows of a (token, kv head) are one contiguous block, so the pass streams.  A warp keeps the
+// slots of its next row pair on the way into its own part of shared memory while it combines the present one
+// (cp.async; a lane reads only what it copied itself, so there is nothing to synchronise), and has the mask of
+// the pair after that: 96 to 192 KB in flight per SM without a gap.
+// Measured at 65 536 tokens x 64 heads x 16 slots (17.4 GB): 2.70 ms = 6.4 TB/s, 98 % of the copy bandwidth; with one
+// row pair per warp and CTA, loaded into registers, it was 3.32 ms (no load was in flight while a warp combined).
+// Slots that were not computed are not read.
 // ------------------------------------------------------------------------------------------
 template <int KBN>
-__global__ void __launch_bounds__(256)
+struct MergeCfg {
+  static constexpr int STAGE = KBN * 512;                     // one row pair: KBN slots x 2 rows x 256 bytes
+  static constexpr int WARPS = 192 * 1024 / (2 * STAGE);      // two stages per warp fill 192 KB
+  static constexpr int SMEM = WARPS * 2 * STAGE;
+  static constexpr int LPL = KBN > 16 ? 2 : 1;                // slots whose LSE a lane of the half warp holds
+};
+
+template <int KBN>
+__global__ void __launch_bounds__(MergeCfg<KBN>::WARPS * 32, 1)
 sparse_merge_kernel(const __nv_bfloat16* __restrict__ po, const float* __restrict__ pl, const int32_t* __restrict__ vmask,
-                    __nv_bfloat16* __restrict__ out, float* __restrict__ lse_out, int kbn, int total_q, int num_heads,
-                    int num_kv_heads, int64_t out_stride_tok, int64_t out_stride_head, float out_scale) {
-  const int l16 = threadIdx.x & 15;
-  const int G = num_heads / num_kv_heads;
-  const int64_t n_idx = static_cast<int64_t>(total_q) * num_heads;
-  for (int64_t idx = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 4) + (threadIdx.x >> 4); idx < n_idx;
-       idx += static_cast<int64_t>(gridDim.x) * (blockDim.x >> 4)) {
-  const int t = static_cast<int>(idx / num_heads), h = static_cast<int>(idx % num_heads);
-  const int kvh = h / G, g = h % G;
-  const int64_t row = idx;
-  const int64_t tk = static_cast<int64_t>(t) * num_kv_heads + kvh;
-  const uint32_t mask = static_cast<uint32_t>(__ldg(vmask + tk));
-  const int64_t prow0 = tk * kbn * G + g;                   // slot s of this row: prow0 + s * G
-  const int piece = l16 ^ (g & 7);                          // the attention kernel stores a row's 16-byte pieces XOR-ed with (head & 7)
-  float lse[KBN];
-  uint4 raw[KBN];
-  float mx = -INFINITY;
+                    __nv_bfloat16* __restrict__ out, float* __restrict__ lse_out, int kbn, int n_rows, int num_heads,
+                    int g_shift, int64_t out_stride_tok, int64_t out_stride_head, float out_scale) {
+  using C = MergeCfg<KBN>;
+  extern __shared__ __align__(128) unsigned char s_merge[];
+  const int lane = threadIdx.x & 31, l16 = lane & 15;
+  const unsigned char* mine = s_merge + (threadIdx.x >> 5) * (2 * C::STAGE) + lane * 16;
+  const uint32_t mine_s = smem_u32(mine);
+  const int G = 1 << g_shift;
+  const int step = gridDim.x * C::WARPS * 2;
+  auto mask_of = [&](int row) -> uint32_t { return row < n_rows ? static_cast<uint32_t>(__ldg(vmask + (row >> g_shift))) : 0u; };
+  auto prow_of = [&](int row) -> int64_t { return static_cast<int64_t>(row >> g_shift) * (kbn << g_shift) + (row & (G - 1)); };
+  float lse[2][C::LPL];
+  // request one row pair into a stage: the slots in `mask`, this lane's LSEs
+  auto request = [&](int row, uint32_t mask, int stage) {
+    const int64_t prow0 = prow_of(row);
+    const unsigned char* src = reinterpret_cast<const unsigned char*>(po) + prow0 * (kHeadDim * 2) +
+                               ((l16 ^ (row & (G - 1) & 7)) << 4);      // the attention kernel stores a row's 16-byte pieces XOR-ed with (head & 7)
 #pragma unroll
-  for (int s = 0; s < KBN; ++s) {
-    const bool have = s < kbn && ((mask >> s) & 1u);
-    const int64_t prow = prow0 + static_cast<int64_t>(s < kbn ? s : 0) * G;   // always a readable row; unused if !have
-    raw[s] = *reinterpret_cast<const uint4*>(po + prow * kHeadDim + piece * 8);
-    const float l = __ldg(pl + prow);
-    lse[s] = have ? l : -INFINITY;
-    mx = fmaxf(mx, lse[s]);
-  }
-  const float mxs = (mx == -INFINITY) ? 0.f : mx;
-  // two columns per packed FMA; a bf16 pair widens with one shift and one mask
-  uint64_t acc2[4];
+    for (int s = 0; s < KBN; ++s)
+      if ((mask >> s) & 1u) cp_async16(mine_s + stage * C::STAGE + s * 512, src + static_cast<int64_t>(s << g_shift) * (kHeadDim * 2), true);
+    cp_async_commit();
 #pragma unroll
-  for (int c = 0; c < 4; ++c) acc2[c] = f2_pack(0.f, 0.f);
-  float sw = 0.f;
-#pragma unroll
-  for (int s = 0; s < KBN; ++s) {
-    const float w = lse[s] != -INFINITY ? __expf(lse[s] - mxs) : 0.f;
-    if (w != 0.f) {                                          // value select after an unconditional load
-      sw += w;
-      const uint64_t w2 = f2_pack(w, w);
-      const uint32_t* r4 = reinterpret_cast<const uint32_t*>(&raw[s]);
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        acc2[c] = f2_fma(f2_pack(__uint_as_float(r4[c] << 16), __uint_as_float(r4[c] & 0xffff0000u)), w2, acc2[c]);
+    for (int i = 0; i < C::LPL; ++i) {
+      const int s = l16 + 16 * i;
+      lse[stage][i] = (s < KBN && ((mask >> s) & 1u)) ? __ldg(pl + prow0 + (s << g_shift)) : -INFINITY;
     }
-  }
-  float acc[8];
+  };
+  // combine one row pair out of a stage
+  auto combine = [&](int row, int stage) {
+    float mx = lse[stage][0];
+    if constexpr (C::LPL == 2) mx = fmaxf(mx, lse[stage][1]);
 #pragma unroll
-  for (int c = 0; c < 4; ++c) f2_unpack(acc2[c], acc[2 * c], acc[2 * c + 1]);
-  const float sc = sw > 0.f ? out_scale / sw : 0.f;
-  __nv_bfloat16* dst = out + static_cast<int64_t>(t) * out_stride_tok + static_cast<int64_t>(h) * out_stride_head + l16 * 8;
-  uint4 pk;
-  pk.x = pack2<false>(acc[0] * sc, acc[1] * sc);
-  pk.y = pack2<false>(acc[2] * sc, acc[3] * sc);
-  pk.z = pack2<false>(acc[4] * sc, acc[5] * sc);
-  pk.w = pack2<false>(acc[6] * sc, acc[7] * sc);
-  *reinterpret_cast<uint4*>(dst) = pk;
-  if (lse_out && l16 == 0) lse_out[row] = sw > 0.f ? mxs + __logf(sw) : -INFINITY;
+    for (int d = 8; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
+    const float mxs = (mx == -INFINITY) ? 0.f : mx;
+    float wl[C::LPL];
+#pragma unroll
+    for (int i = 0; i < C::LPL; ++i) wl[i] = lse[stage][i] != -INFINITY ? __expf(lse[stage][i] - mxs) : 0.f;
+    // two columns per packed FMA; a bf16 pair widens with one shift and one mask
+    uint64_t acc2[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc2[c] = f2_pack(0.f, 0.f);
+    float sw = 0.f;
+#pragma unroll
+    for (int s = 0; s < KBN; ++s) {
+      const float w = __shfl_sync(0xffffffffu, wl[s >> 4], (lane & 16) | (s & 15));
+      const uint4 raw = *reinterpret_cast<const uint4*>(mine + stage * C::STAGE + s * 512);
+      if (w != 0.f) {                                         // a slot that was not computed holds anything
+        sw += w;
+        const uint64_t w2 = f2_pack(w, w);
+        const uint32_t r4[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          acc2[c] = f2_fma(f2_pack(__uint_as_float(r4[c] << 16), __uint_as_float(r4[c] & 0xffff0000u)), w2, acc2[c]);
+      }
+    }
+    const float sc = sw > 0.f ? out_scale / sw : 0.f;
+    if (row >= n_rows) return;
+    const int t = row / num_heads, h = row - t * num_heads;
+    __nv_bfloat16* dst = out + static_cast<int64_t>(t) * out_stride_tok + static_cast<int64_t>(h) * out_stride_head + l16 * 8;
+    uint32_t w[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      float a, b;
+      f2_unpack(acc2[c], a, b);
+      w[c] = pack2<false>(a * sc, b * sc);
+    }
+    *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+    if (lse_out && l16 == 0) lse_out[row] = sw > 0.f ? mxs + __logf(sw) : -INFINITY;
+  };
+
+  const int first = (blockIdx.x * C::WARPS + static_cast<int>(threadIdx.x >> 5)) * 2;   // the same for the whole warp
+  const int half = lane >> 4;
+  uint32_t mask = mask_of(first + half);
+  request(first + half, mask, 0);
+  mask = mask_of(first + step + half);
+  for (int64_t base = first; base < n_rows; base += 2 * static_cast<int64_t>(step)) {
+#pragma unroll
+    for (int st = 0; st < 2; ++st) {                          // static stage indices
+      const int64_t row = base + static_cast<int64_t>(st) * step + half;
+      if (row - half >= n_rows) break;
+      const int64_t next = row + step;
+      request(static_cast<int>(min(next, static_cast<int64_t>(n_rows))), mask, st ^ 1);   // past the end: mask is 0
+      mask = mask_of(static_cast<int>(min(next + step, static_cast<int64_t>(n_rows))));
+      cp_async_wait<1>();
+      combine(static_cast<int>(row), st);
+    }
   }
 }
 
@@ -756,6 +799,29 @@ sparse_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
   }
 }
 
+template <int KBN>
+int launch_merge(const MsaFmhaParams& p, const Ws& w, cudaStream_t stream) {
+  using C = MergeCfg<KBN>;
+  static bool attr_done[16] = {};
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return MSA_ERR_LAUNCH;
+  if (dev >= 16 || !attr_done[dev]) {
+    if (cudaFuncSetAttribute(sparse_merge_kernel<KBN>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
+      return MSA_ERR_LAUNCH;
+    if (dev < 16) attr_done[dev] = true;
+  }
+  const int rows = p.total_q * p.num_qo_heads;                 // fits: fmha_sparse_tc_supported bounds rows x slots
+  const int per_cta = C::WARPS * 2;
+  const int blocks = min(sms, (rows + per_cta - 1) / per_cta);
+  int g_shift = 0;
+  while ((p.num_kv_heads << g_shift) < p.num_qo_heads) ++g_shift;   // G divides 128
+  sparse_merge_kernel<KBN><<<blocks, C::WARPS * 32, C::SMEM, stream>>>(
+      w.partial_o, w.partial_lse, w.vmask, static_cast<__nv_bfloat16*>(p.out), p.lse, p.kv_block_num, rows, p.num_qo_heads,
+      g_shift, p.out_stride_tok, p.out_stride_head, p.out_scale);
+  return cudaGetLastError() == cudaSuccess ? MSA_OK : MSA_ERR_LAUNCH;
+}
+
 }  // namespace
 }  // namespace sparse_tc
 
@@ -876,19 +942,9 @@ int fmha_sparse_tc_launch(const MsaFmhaParams& p, cudaStream_t stream) {
   // second stream with a small grid while the attention kernel works on head k + 1 was tried: an SM
   // sustains ~60 GB/s of gathered reads with its registers as the only landing space, so the merge
   // needs a third of the SMs to keep up and the attention kernel loses more than the merge gains.)
-  const int64_t rows = static_cast<int64_t>(p.total_q) * p.num_qo_heads;
-  const int64_t blocks = (rows + 15) / 16;
-  if (blocks > 0x7fffffffLL) return MSA_ERR_TOO_LARGE;
-  __nv_bfloat16* outp = static_cast<__nv_bfloat16*>(p.out);
-#define MSA_MERGE(KK)                                                                                             \
-  sparse_merge_kernel<KK><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(                                    \
-      w.partial_o, w.partial_lse, w.vmask, outp, p.lse, p.kv_block_num, p.total_q, p.num_qo_heads, p.num_kv_heads, \
-      p.out_stride_tok, p.out_stride_head, p.out_scale)
-  if (p.kv_block_num <= 8) MSA_MERGE(8);
-  else if (p.kv_block_num <= 16) MSA_MERGE(16);
-  else MSA_MERGE(32);
-#undef MSA_MERGE
-  return cudaGetLastError() == cudaSuccess ? MSA_OK : MSA_ERR_LAUNCH;
+  if (p.kv_block_num <= 8) return launch_merge<8>(p, w, stream);
+  if (p.kv_block_num <= 16) return launch_merge<16>(p, w, stream);
+  return launch_merge<32>(p, w, stream);
 }
 
 }  // namespace msa
