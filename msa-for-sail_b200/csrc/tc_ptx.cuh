@@ -79,6 +79,26 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// ------------------------------------------------------------------ launch control
+// Ask for a CTA of this grid that has not started; the 16-byte answer and a complete_tx of 16 bytes on `bar` follow.
+// Not to be called again once an answer was "none".
+__device__ __forceinline__ void clc_try_cancel(uint32_t answer, uint32_t bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+               ::"r"(answer), "r"(bar) : "memory");
+}
+// blockIdx.x of the CTA that will not be launched because this one does its work, or -1
+__device__ __forceinline__ int clc_first_ctaid(uint32_t answer) {
+  int x;
+  asm volatile(
+      "{\n\t.reg .b128 a;\n\t.reg .pred p;\n\t"
+      "ld.shared.b128 a, [%1];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, a;\n\t"
+      "mov.b32 %0, -1;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, a;\n\t}"
+      : "=r"(x) : "r"(answer) : "memory");
+  return x;
+}
+
 // ------------------------------------------------------------------ TMA (tiled, no cluster broadcast)
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1,
                                             int c2) {
