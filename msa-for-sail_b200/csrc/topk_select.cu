@@ -7,13 +7,12 @@
 // upstream order-preserving float->uint map (sparse_topk_select.cuh:186-213); pages forced by
 // force_begin / force_end rank as FLT_MAX (kForcedOrd there).
 //
-// Layout of the work: a CTA owns 32 consecutive tokens of one head; its lanes read 32
-// consecutive tokens (one coalesced 128-byte line per page row for fp32), its SL warps scan
-// interleaved blocks of TOPK pages.  Each thread keeps its TOPK best keys sorted in registers and
-// folds in TOPK new keys at a time with bitonic compare-exchange networks (branch-free: rows of a
-// warp never diverge).  The SL partial lists are merged through shared memory with the same network.
-// HBM traffic is one read of the valid part of the score tensor plus the index write; no
-// transpose workspace (upstream needs one, api.py:1818-1821).
+// Layout of the work for prefill-sized inputs: a CTA owns 32 consecutive tokens of one head; its lanes read 32
+// consecutive tokens (one coalesced 128-byte line per page row for fp32), its SL warps share the pages, a thread per
+// row and warp.  Two kernels of that layout: topk_threshold_kernel finds the TOPK-th best score of a row with 32-bit
+// keys and picks the pages in a second scan; topk_select_kernel (bf16 scores) keeps whole keys, score and page, in one
+// 32-bit word and needs one scan.  No transpose workspace (upstream needs one, api.py:1818-1821).
+// Decode-sized inputs: topk_row_kernel, a CTA per row.
 #include "common.cuh"
 #include "nvtx_range.h"
 
@@ -32,14 +31,10 @@ __device__ __forceinline__ uint32_t ord_key(float v) {
   return v != v ? 0xFFFFFFFFu : key;
 }
 
-// Keys of the thread-per-row kernel.  Keys are unique (the page is part of them), hence a strict total order:
-// no tie handling anywhere.
-//   Key64  (order key << 32 | ~page) in one 64-bit word: a compare-exchange is one 64-bit compare and two
-//          64-bit selects.  (An (order key, page) pair in two 32-bit registers, 3 compares + 4 selects per
-//          exchange, measured 116-121 us against 101 us at 65 536 rows x 256 pages of fp32 scores.)
-//   Key1   bf16 scores: the upper half of the order key is exact for them, so (key16 << 16 | ~page16) is one
-//          32-bit word and an exchange is one max and one min.  Not used with forced pages, which rank as the
-//          fp32 maximum -- a score bf16 cannot tell from its own largest finite value -- nor beyond 65 535 pages.
+// Key of topk_select_kernel: bf16 scores only, where the upper half of the order key is exact, so
+// (key16 << 16 | ~page16) is one unique 32-bit word (no tie handling anywhere) and a compare-exchange is one max and
+// one min.  Not used with forced pages, which rank as the fp32 maximum -- a score bf16 cannot tell from its own largest
+// finite value -- nor beyond 65 535 pages.
 struct Key1 {
   uint32_t k;
   static __device__ __forceinline__ Key1 none() { return {0u}; }
@@ -48,42 +43,31 @@ struct Key1 {
   }
   __device__ __forceinline__ bool is_none() const { return k == 0u; }
   __device__ __forceinline__ uint32_t page() const { return 0xffffu - (k & 0xffffu); }
-  static __device__ __forceinline__ void order(Key1& a, Key1& b) {
-    const uint32_t hi = max(a.k, b.k), lo = min(a.k, b.k);
-    a.k = hi; b.k = lo;
-  }
-  static __device__ __forceinline__ Key1 best(const Key1& a, const Key1& b) { return {max(a.k, b.k)}; }
 };
+__device__ __forceinline__ void order(Key1& a, Key1& b) {
+  const uint32_t hi = max(a.k, b.k), lo = min(a.k, b.k);
+  a.k = hi; b.k = lo;
+}
+__device__ __forceinline__ Key1 best(const Key1& a, const Key1& b) { return {max(a.k, b.k)}; }
+__device__ __forceinline__ void order(uint32_t& a, uint32_t& b) {
+  const uint32_t hi = max(a, b), lo = min(a, b);
+  a = hi; b = lo;
+}
+__device__ __forceinline__ uint32_t best(uint32_t a, uint32_t b) { return max(a, b); }
 
-struct Key64 {
-  unsigned long long k;
-  static __device__ __forceinline__ Key64 none() { return {0ull}; }
-  static __device__ __forceinline__ Key64 make(uint32_t ord, int page) {
-    return {(static_cast<unsigned long long>(ord) << 32) | (0xffffffffu - static_cast<uint32_t>(page))};
-  }
-  __device__ __forceinline__ bool is_none() const { return (k >> 32) == 0ull; }
-  __device__ __forceinline__ uint32_t page() const { return 0xffffffffu - static_cast<uint32_t>(k); }
-  static __device__ __forceinline__ void order(Key64& a, Key64& b) {
-    const bool sw = b.k > a.k;
-    const unsigned long long hi = sw ? b.k : a.k, lo = sw ? a.k : b.k;
-    a.k = hi; b.k = lo;
-  }
-  static __device__ __forceinline__ Key64 best(const Key64& a, const Key64& b) { return {b.k > a.k ? b.k : a.k}; }
-};
-
-// descending bitonic sort of N keys / merge of a descending list into the sorted top-N list (static
-// register indices, no data-dependent branch: the 32 rows a warp owns never diverge)
+// Descending sort of N keys (odd-even merge sort: 63 exchanges for 16 keys) / merge of a descending list into the
+// sorted top-N list.  Static register indices, no data-dependent branch: the 32 rows a warp owns never diverge.
 template <int N, typename K>
 __device__ __forceinline__ void net_sort_desc(K (&v)[N]) {
 #pragma unroll
-  for (int k = 2; k <= N; k <<= 1) {
+  for (int p = 1; p < N; p <<= 1) {
 #pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1) {
+    for (int k = p; k > 0; k >>= 1) {
 #pragma unroll
-      for (int i = 0; i < N; ++i) {
-        const int l = i ^ j;
-        if (l > i) {
-          if ((i & k) == 0) K::order(v[i], v[l]); else K::order(v[l], v[i]);
+      for (int j = k % p; j + k < N; j += 2 * k) {
+#pragma unroll
+        for (int i = 0; i < k; ++i) {
+          if (i + j + k < N && (i + j) / (2 * p) == (i + j + k) / (2 * p)) order(v[i + j], v[i + j + k]);
         }
       }
     }
@@ -92,21 +76,156 @@ __device__ __forceinline__ void net_sort_desc(K (&v)[N]) {
 template <int N, typename K>
 __device__ __forceinline__ void net_merge_desc(K (&key)[N], const K (&v)[N]) {
 #pragma unroll
-  for (int i = 0; i < N; ++i) key[i] = K::best(key[i], v[N - 1 - i]);     // bitonic now
+  for (int i = 0; i < N; ++i) key[i] = best(key[i], v[N - 1 - i]);     // bitonic now
 #pragma unroll
   for (int j = N >> 1; j > 0; j >>= 1) {
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       const int l = i ^ j;
-      if (l > i) K::order(key[i], key[l]);
+      if (l > i) order(key[i], key[l]);
     }
   }
 }
 
-template <int TOPK, typename T, typename K>
+// Two scans of a row's pages.  The first keeps the TOPK largest order keys -- the scores alone, 32 bits: an exchange
+// is a max and a min, where (score, page) in one 64-bit word costs a 64-bit compare and two selects of pairs -- and
+// leaves the threshold, the TOPK-th best key.  The second scan, in page order, takes every page above the threshold
+// and the first of those at it, as many as fit: exactly the order (key desc, page asc), and the pages come out
+// ascending without a sort.  The scores of the second scan come from L2.
+// Measured on fp32 scores, kernel alone: 65 536 rows x 256 pages 103 -> 52 us, 32 768 rows x 769 pages 133 -> 65 us
+// (64-bit keys in one scan before); 256 tokens x 4 heads x 256 pages 18.5 us (a CTA per row) -> 7.5 us.
+// FORCED: some pages rank as FLT_MAX whatever their score.
+template <int TOPK, typename T, bool FORCED>
+__global__ void __launch_bounds__(512)
+topk_threshold_kernel(const T* __restrict__ scores, int32_t* __restrict__ out, int num_heads, int max_k_tiles,
+                      int total_q, int nvp, int force_begin, int force_end_start, int slices) {
+  extern __shared__ uint32_t s_lists[];             // [slices][TOPK][32]: keys of the first scan, pages of the second
+  __shared__ uint32_t s_threshold[32], s_count[16 * 32];
+  __shared__ int s_quota[32];
+  constexpr uint32_t kTie = 0x80000000u;
+  constexpr float kMax = 3.402823466e38f;
+  const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
+  const int tok_blocks = (total_q + 31) / 32;
+  const int head = blockIdx.x / tok_blocks;
+  const int t = (blockIdx.x % tok_blocks) * 32 + lane;
+  const bool live = t < total_q;
+  // a lane past the last token walks the last one: its loads are valid, its result is not stored
+  const T* base = scores + static_cast<size_t>(head) * max_k_tiles * total_q + min(t, total_q - 1);
+  uint32_t* mine = s_lists + sl * (TOPK * 32) + lane;
+  // a contiguous part of the pages per warp, whole blocks of TOPK
+  const int blocks = (nvp + TOPK - 1) / TOPK, per = (blocks + slices - 1) / slices;
+  const int p0 = min(nvp, sl * per * TOPK), p1 = min(nvp, p0 + per * TOPK);
+  // scores of up to N pages from k0 on, all loads before any use; those past p1 are not read
+  auto load = [&](auto& v, int k0) {
+    constexpr int N = sizeof(v) / sizeof(float);
+    const T* ptr = base + static_cast<size_t>(k0) * total_q;
+    if (k0 + N <= p1) {
+#pragma unroll
+      for (int u = 0; u < N; ++u, ptr += total_q) v[u] = static_cast<float>(*ptr);
+    } else {
+#pragma unroll
+      for (int u = 0; u < N; ++u, ptr += total_q) v[u] = k0 + u < p1 ? static_cast<float>(*ptr) : 0.f;
+    }
+    if constexpr (FORCED) {
+#pragma unroll
+      for (int u = 0; u < N; ++u)
+        if (k0 + u < force_begin || k0 + u >= force_end_start) v[u] = kMax;
+    }
+  };
+
+  uint32_t top[TOPK];
+#pragma unroll
+  for (int i = 0; i < TOPK; ++i) top[i] = 0u;       // below every order key
+  for (int k0 = p0; k0 < p1; k0 += TOPK) {
+    float v[TOPK];
+    load(v, k0);
+    uint32_t blk[TOPK];
+#pragma unroll
+    for (int u = 0; u < TOPK; ++u) blk[u] = ord_key(v[u]);
+    if (k0 + TOPK > p1) {
+#pragma unroll
+      for (int u = 0; u < TOPK; ++u)
+        if (k0 + u >= p1) blk[u] = 0u;
+    }
+    net_sort_desc<TOPK, uint32_t>(blk);
+    net_merge_desc<TOPK, uint32_t>(top, blk);
+  }
+  // tree merge of the slices' lists into slice 0 (slices is a power of two)
+  for (int d = 1; d < slices; d <<= 1) {
+    if ((sl & (2 * d - 1)) == d) {
+#pragma unroll
+      for (int i = 0; i < TOPK; ++i) mine[i * 32] = top[i];
+    }
+    __syncthreads();
+    if ((sl & (2 * d - 1)) == 0) {
+      uint32_t o[TOPK];
+#pragma unroll
+      for (int i = 0; i < TOPK; ++i) o[i] = mine[(d * TOPK + i) * 32];
+      net_merge_desc<TOPK, uint32_t>(top, o);
+    }
+  }
+  if (sl == 0) {
+    int above = 0;
+#pragma unroll
+    for (int i = 0; i < TOPK; ++i) above += top[i] > top[TOPK - 1] ? 1 : 0;
+    s_threshold[lane] = top[TOPK - 1];
+    s_quota[lane] = TOPK - above;                   // pages to take among those at the threshold
+  }
+  __syncthreads();
+  // The second scan compares scores: the order key of a number grows with it, -0 and +0 compare equal, and a NaN is
+  // above every number (not <=) but ties with a NaN threshold.
+  const uint32_t tkey = s_threshold[lane];
+  const bool t_nan = tkey == 0xffffffffu;
+  const float thr = t_nan ? __int_as_float(0x7fffffff) : __uint_as_float(tkey & 0x80000000u ? tkey ^ 0x80000000u : ~tkey);
+  const int quota = s_quota[lane];
+  int n = 0, ties = 0;
+  for (int k0 = p0; k0 < p1; k0 += 16) {
+    float v[16];
+    load(v, k0);
+    uint32_t above = 0, level = 0;                  // bit u: page k0 + u
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      if (!(v[u] <= thr)) above |= 1u << u;
+      if (v[u] == thr || (t_nan && v[u] != v[u])) level |= 1u << u;
+    }
+    if (t_nan) above = 0;
+    uint32_t take = above | level;
+    if (k0 + 16 > p1) take &= (1u << (p1 - k0)) - 1u;
+    while (take != 0) {
+      const int u = __ffs(take) - 1;
+      take &= take - 1;
+      const bool tie = (level >> u) & 1u;
+      if (tie && ties >= quota) continue;           // at most TOPK of a row in all: fewer above than TOPK, quota ties
+      mine[n * 32] = static_cast<uint32_t>(k0 + u) | (tie ? kTie : 0u);
+      ++n;
+      ties += tie ? 1 : 0;
+    }
+  }
+  s_count[sl * 32 + lane] = static_cast<uint32_t>(n - ties) << 16 | static_cast<uint32_t>(ties);
+  __syncthreads();
+  // slice s of a row puts its pages behind those of the slices before it, whose ties use up the quota first
+  int pos = 0, left = quota;
+  for (int s2 = 0; s2 < sl; ++s2) {
+    const uint32_t c = s_count[s2 * 32 + lane];
+    const int use = min(left, static_cast<int>(c & 0xffffu));
+    pos += static_cast<int>(c >> 16) + use;
+    left -= use;
+  }
+  if (!live) return;
+  int32_t* dst = out + (static_cast<size_t>(t) * num_heads + head) * TOPK;
+  for (int i = 0; i < n; ++i) {
+    const uint32_t page = mine[i * 32];
+    const bool tie = (page & kTie) != 0;
+    if (!tie || left > 0) dst[pos++] = static_cast<int32_t>(page & ~kTie);
+    if (tie) --left;
+  }
+}
+
+template <int TOPK, typename T>
 __global__ void __launch_bounds__(256)
 topk_select_kernel(const T* __restrict__ scores, int32_t* __restrict__ out, int num_heads, int max_k_tiles,
-                   int total_q, int nvp, int force_begin, int force_end_start, int slices) {
+                   int total_q, int nvp, int slices) {
+  using K = Key1;
   extern __shared__ __align__(8) unsigned char s_raw[];
   K* s_keys = reinterpret_cast<K*>(s_raw);          // [slices][32][TOPK]
   const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
@@ -130,8 +249,7 @@ topk_select_kernel(const T* __restrict__ scores, int32_t* __restrict__ out, int 
 #pragma unroll
       for (int u = 0; u < TOPK; ++u) {
         const int kk = k0 + u;
-        const bool forced = kk < force_begin || kk >= force_end_start;
-        blk[u] = kk < nvp ? K::make(forced ? kForcedOrd : ord_key(v[u]), kk) : K::none();
+        blk[u] = kk < nvp ? K::make(ord_key(v[u]), kk) : K::none();
       }
       net_sort_desc<TOPK, K>(blk);
       net_merge_desc<TOPK, K>(top, blk);
@@ -281,7 +399,10 @@ int launch(const T* scores, int32_t* out, int H, int K, int T_, int nvp, int fb,
     return cudaGetLastError() == cudaSuccess ? MSA_OK : MSA_ERR_LAUNCH;
   }
   const int fe_start = fe <= nvp ? nvp - fe : 0;
-  if (rows <= 2048 && nvp <= 256 * 32) {                     // decode-sized: a CTA per row
+  const bool one_word = sizeof(T) == 2 && fb == 0 && fe == 0 && nvp <= 65535;      // bf16 scores, nothing forced
+  // Decode-sized: a CTA per row, where fewer than 32 tokens would leave lanes of a thread-per-row kernel idle (32
+  // tokens x 1 head x 1 024 pages on a CTA per row: 7.4 us).
+  if ((T_ < 32 || one_word) && rows <= 2048 && nvp <= 256 * 32) {
     if (nvp <= 256 * 4)
       topk_row_kernel<TOPK, 4, T><<<static_cast<unsigned>(rows), 256, 0, stream>>>(scores, out, H, K, T_, nvp, fb, fe_start);
     else if (nvp <= 256 * 8)
@@ -292,20 +413,20 @@ int launch(const T* scores, int32_t* out, int H, int K, int T_, int nvp, int fb,
   }
   const int tok_blocks = (T_ + 31) / 32;
   const long long ctas = static_cast<long long>(tok_blocks) * H;
-  // enough slices to put ~16 warps on every SM, bounded by the pages there are to scan
-  int slices = 1;
-  while (slices < 8 && ctas * slices < 148LL * 16 && nvp / (slices * 2) >= 2 * TOPK) slices *= 2;
   if (ctas > 0x7fffffffLL) return MSA_ERR_TOO_LARGE;
-  const bool one_word = sizeof(T) == 2 && fb == 0 && fe == 0 && nvp <= 65535;      // bf16 scores, nothing forced
-  const size_t smem = slices > 1 ? static_cast<size_t>(slices) * 32 * TOPK * (one_word ? sizeof(Key1) : sizeof(Key64)) : 0;
   const unsigned grid = static_cast<unsigned>(ctas);
+  // enough slices to put ~16 warps on every SM, bounded by the pages there are to scan
+  const int most = one_word ? 8 : 16, least_blocks = one_word ? 2 : 1;      // blocks of TOPK pages per slice
+  int slices = 1;
+  while (slices < most && ctas * slices < 148LL * 16 && nvp / (slices * 2) >= least_blocks * TOPK) slices *= 2;
+  const size_t smem = static_cast<size_t>(slices) * 32 * TOPK * 4;
   if (one_word) {
-    auto kern = topk_select_kernel<TOPK, T, Key1>;
+    auto kern = topk_select_kernel<TOPK, T>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    kern<<<grid, 32 * slices, smem, stream>>>(scores, out, H, K, T_, nvp, fb, fe_start, slices);
+    kern<<<grid, 32 * slices, smem, stream>>>(scores, out, H, K, T_, nvp, slices);
   } else {
-    auto kern = topk_select_kernel<TOPK, T, Key64>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    auto kern = fb > 0 || fe_start < nvp ? topk_threshold_kernel<TOPK, T, true> : topk_threshold_kernel<TOPK, T, false>;
+    if (smem > 44 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     kern<<<grid, 32 * slices, smem, stream>>>(scores, out, H, K, T_, nvp, fb, fe_start, slices);
   }
   return cudaGetLastError() == cudaSuccess ? MSA_OK : MSA_ERR_LAUNCH;
