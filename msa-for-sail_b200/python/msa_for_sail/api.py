@@ -35,7 +35,7 @@ _STATUS = {}
 
 def _status_word(device):
     """Per-device int32 status word the kernels report bounded-wait timeouts into."""
-    idx = torch.device(device).index or 0
+    idx = (device if isinstance(device, torch.device) else torch.device(device)).index or 0
     if idx not in _STATUS:
         _STATUS[idx] = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx))
     return _STATUS[idx]
@@ -67,7 +67,8 @@ def _ptr(t):
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    # the handle of torch.cuda.current_stream(), without building a Stream object (4 us of a 20 us call)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _dt_code(dtype):
@@ -126,12 +127,15 @@ class PlanInfo(dict):
 # workspace arena (graph-safe callers hand in one fixed uint8 tensor)
 # ----------------------------------------------------------------------------
 
+_ITEM_BYTES = {torch.int32: 4, torch.float32: 4}
+
+
 class _Arena:
     def __init__(self, buf, device):
         self.buf, self.off, self.device = buf, 0, device
 
     def take(self, numel, dtype):
-        item = torch.empty(0, dtype=dtype).element_size()
+        item = _ITEM_BYTES[dtype]
         if self.buf is None:
             return torch.empty(numel, dtype=dtype, device=self.device)
         self.off = (self.off + 255) & ~255
@@ -143,6 +147,30 @@ class _Arena:
         out = self.buf[self.off:end].view(dtype)
         self.off = end
         return out
+
+
+class _Upload:
+    """The int32 arrays of one plan, laid out in one block (256 bytes apart) and copied to the device at once: a copy
+    from pageable memory waits for the stream, and a plan has up to ten arrays."""
+
+    def __init__(self):
+        self.parts, self.total = [], 0                     # (key, offset, array, numel)
+
+    def add(self, key, values, numel=None):
+        a = np.asarray(values, dtype=np.int32).reshape(-1)
+        off = (self.total + 63) & ~63
+        self.total = off + (a.size if numel is None else numel)
+        self.parts.append((key, off, a, self.total - off))
+
+    def run(self, arena, info):
+        """Take the block from `arena`, copy, and put a view of every array into `info`."""
+        host = np.empty(self.total, np.int32)
+        for _, off, a, _ in self.parts:
+            host[off:off + a.size] = a
+        block = arena.take(self.total, torch.int32)
+        block.copy_(torch.from_numpy(host))
+        for key, off, _, n in self.parts:
+            info[key] = block[off:off + n]
 
 
 def _workspace_bytes(batch, total_q, num_qo_heads, splits, sparse):
@@ -174,7 +202,8 @@ def allocate_graph_workspace(batch_size, num_qo_heads, num_kv_heads=-1,
 
 def _to_int_list(t):
     if isinstance(t, torch.Tensor):
-        return [int(x) for x in t.detach().cpu().reshape(-1).tolist()]
+        v = t.detach().cpu().reshape(-1).tolist()
+        return [int(x) for x in v] if t.is_floating_point() else v
     return [int(x) for x in t]
 
 
@@ -287,31 +316,26 @@ def _fmha_sail_plan(
 
     arena = _Arena(given_workspace, dev)
 
-    def upload(values, n=None):
-        a = np.asarray(values, dtype=np.int32)
-        t = arena.take(a.size if n is None else n, torch.int32)
-        if a.size:
-            t[:a.size].copy_(torch.from_numpy(a), non_blocking=False)
-        return t
-
+    up = _Upload()
     qo_start = np.zeros(batch + 1, np.int32); qo_start[1:] = np.cumsum(qo_lens)
     kv_start = np.zeros(batch + 1, np.int32); kv_start[1:] = np.cumsum(kv_lens)
+    a_q, a_k, a_o = (np.asarray(v, np.int32) for v in (qo_lens, kv_lens, offs))
     info = PlanInfo()
-    info["qo_segment_offsets"] = upload(qo_start)
-    info["kv_segment_offsets"] = upload(kv_start)
-    info["qo_segment_lens"] = upload(qo_lens)
-    info["kv_segment_lens"] = upload(kv_lens)
-    info["qo_offset"] = upload(offs)
+    up.add("qo_segment_offsets", qo_start)
+    up.add("kv_segment_offsets", kv_start)
+    up.add("qo_segment_lens", a_q)
+    up.add("kv_segment_lens", a_k)
+    up.add("qo_offset", a_o)
     if page_size > 0:
+        pages_per = (a_k + (page_size - 1)) // page_size
         indptr = np.zeros(batch + 1, np.int32)
-        indptr[1:] = np.cumsum([(k + page_size - 1) // page_size for k in kv_lens])
-        info["kv_page_indptr"] = upload(indptr)
+        indptr[1:] = np.cumsum(pages_per)
+        up.add("kv_page_indptr", indptr)
     else:
         info["kv_page_indptr"] = None
 
-    work = None
     num_work = 0
-    splits_per_row = None
+    info["work"] = info["num_kv_splits_per_row"] = None
     if is_sparse:
         items = total_q * hkv
         if num_kv_splits >= 1:
@@ -325,17 +349,15 @@ def _fmha_sail_plan(
             splits = 1
             while splits * 2 <= min(kv_block_num, 8) and items * splits < 2 * num_sms:
                 splits *= 2
-        info["token_batch"] = upload(np.repeat(np.arange(batch, dtype=np.int32), qo_lens))
-        pages_per = [(kl + page_size - 1) // page_size for kl in kv_lens]
-        info["page_batch"] = upload(np.repeat(np.arange(batch, dtype=np.int32), pages_per))
-        info["num_logical_pages"] = int(sum(pages_per))
+        up.add("token_batch", np.repeat(np.arange(batch, dtype=np.int32), a_q))
+        up.add("page_batch", np.repeat(np.arange(batch, dtype=np.int32), pages_per))
+        info["num_logical_pages"] = int(pages_per.sum())
         info["sparse_ws"] = None
         # page-major path pays off once several tokens share a page
-        info["sparse_tc_preferred"] = (sum(pages_per) > 0 and total_q * kv_block_num >= 8 * sum(pages_per)
-                                       and total_q >= 256)
+        info["sparse_tc_preferred"] = (info["num_logical_pages"] > 0 and total_q >= 256
+                                       and total_q * kv_block_num >= 8 * info["num_logical_pages"])
     else:
         info["token_batch"] = None
-        a_q = np.asarray(qo_lens, np.int32); a_k = np.asarray(kv_lens, np.int32); a_o = np.asarray(offs, np.int32)
         args = _lib.MsaPlanArgs(
             a_q.ctypes.data, a_k.ctypes.data, a_o.ctypes.data, batch, num_qo_heads, hkv, block_m, pack,
             num_kv_splits if num_kv_splits >= 1 else -128, num_sms, 0)
@@ -353,12 +375,10 @@ def _fmha_sail_plan(
             break
         num_work = n
         splits = int(max_splits.value)
-        work = arena.take(max(1, n) * 8, torch.int32)
-        if n:
-            work[:n * 8].copy_(torch.from_numpy(host[:n].reshape(-1)))
+        up.add("work", host[:n], max(1, n) * 8)
         info["_work_host"] = host[:n]
         if splits > 1:
-            splits_per_row = upload(spr[:total_q])
+            up.add("num_kv_splits_per_row", spr[:total_q])
         # second work list in 256-row items for the tcgen05 prefill kernel (q and k both bf16 or
         # both e4m3, unsplit, one query head per row tile, ragged K/V or 128-key pages)
         info["work_tc"], info["num_work_tc"] = None, 0
@@ -372,13 +392,13 @@ def _fmha_sail_plan(
             n_tc = _lib.check(_lib.lib.msa_plan_dense(ctypes.byref(args_tc), host_tc.ctypes.data, cap_tc,
                                                       None, None), "msa_plan_dense")
             if n_tc:
-                wt = arena.take(n_tc * 8, torch.int32)
-                wt.copy_(torch.from_numpy(host_tc[:n_tc].reshape(-1)))
-                info["work_tc"], info["num_work_tc"] = wt, n_tc
+                up.add("work_tc", host_tc[:n_tc])
+                info["num_work_tc"] = n_tc
                 # with far too few items to fill the GPU the split-KV plan of the generic kernel wins
                 # (a 256-row tcgen05 item runs about three times as fast as the same rows there)
                 info["tc_preferred"] = splits == 1 or n_tc * 2 >= num_sms
 
+    up.run(arena, info)
     if splits > 1:
         info["workspace_o"] = arena.take(splits * total_q * orig_num_qo_heads * 128, torch.float32)
         info["workspace_lse"] = arena.take(splits * total_q * orig_num_qo_heads, torch.float32)
@@ -394,10 +414,8 @@ def _fmha_sail_plan(
     info.update({
         "qo_tile_size": block_m,
         "kv_tile_size": KV_TILE,
-        "work": work,
         "num_work": num_work,
         "num_kv_splits": splits,
-        "num_kv_splits_per_row": splits_per_row,
         "max_qo_len": max_qo,
         "predicted_speedup": 1.0,
         "max_k_tiles": max_k_tiles,
@@ -890,8 +908,8 @@ def _decode_prefix(qo_segment_lens, sparse):
     """Length of the leading run of short-query (decode) batch items when the batch also holds a
     long-query (prefill) item, else 0.  Items are expected decode-first, as upstream's mixed
     batches are (api.py:1555-1575)."""
-    long_items = (qo_segment_lens > _prefill_qlen_threshold(sparse)).nonzero(as_tuple=False)
-    return int(long_items[0, 0].item()) if long_items.numel() else 0
+    threshold = _prefill_qlen_threshold(sparse)
+    return next((i for i, n in enumerate(qo_segment_lens.tolist()) if n > threshold), 0)
 
 
 def fmha_sail_plan(
