@@ -31,6 +31,31 @@ __device__ __forceinline__ int chk(int v, int lo, int hi, int32_t* status) {
 __device__ __forceinline__ int chk(int v, int, int, int32_t*) { return v; }
 #endif
 
+// ---- kernels of one stream without a gap between them ----
+// A kernel launched with launch_chained() may start while the kernel before it in the stream still runs: once every CTA of
+// that one has called chain_begin() or ended.  chain_begin() comes before anything that touches global memory: it waits
+// until the kernel before has completed and its writes are visible (at once if there is nothing to wait for), then
+// lets the next kernel of the stream come up in the same way.  So the order of all memory accesses is that of the
+// stream, and only the launch and the start of the CTAs overlap.
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  // Under capture the launches stay plain: with programmatic edges the replay of a six-kernel decode graph took 86.5 us
+  // against 77 us.
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(stream, &capture);
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = capture == cudaStreamCaptureStatusNone ? 1 : 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }

@@ -149,6 +149,7 @@ decode_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
   const int G = p.pack;
   const int h_r = p.num_qo_heads / p.num_kv_heads;
 
+  chain_begin();
   // ---------------- work item ----------------
   int b, head0, tb, te, split, i_base, ntok;
   int blk_first = -1;                       // sparse: this lane's entry of the selected-page list, fetched early
@@ -866,8 +867,7 @@ int fmha_decode_tc_launch(const MsaFmhaParams& p, cudaStream_t stream) {
       cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (dev < 16) attr_done[dev][variant] = true;
   }
-  kern<<<static_cast<unsigned>(grid64), NTHREADS, smem, stream>>>(p, tq, tk, tv);
-  return cudaGetLastError() == cudaSuccess ? MSA_OK : MSA_ERR_LAUNCH;
+  return launch_chained(kern, static_cast<unsigned>(grid64), NTHREADS, smem, stream, p, tq, tk, tv) == cudaSuccess ? MSA_OK : MSA_ERR_LAUNCH;
 }
 
 // CTAs of one decode-kernel variant that fit an SM (what the occupancy calculator reports).

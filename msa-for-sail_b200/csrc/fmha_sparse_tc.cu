@@ -156,6 +156,7 @@ template <bool SCATTER>
 __global__ void __launch_bounds__(256)
 sparse_index_kernel(const IndexArgs a, int32_t* __restrict__ bin_count, int32_t* __restrict__ bin_cursor,
                     int32_t* __restrict__ entries, int32_t* __restrict__ vmask) {
+  chain_begin();
   const int64_t gid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;   // kvh-major, token fastest
   const int64_t n = static_cast<int64_t>(a.total_q) * a.num_kv_heads;
   if (gid >= n) return;
@@ -184,6 +185,7 @@ template <bool SCATTER, int KBN>
 __global__ void __launch_bounds__(256)
 sparse_index_smem_kernel(const IndexArgs a, int32_t* __restrict__ bin_count, int32_t* __restrict__ bin_cursor,
                          int32_t* __restrict__ entries, int32_t* __restrict__ vmask) {
+  chain_begin();
   extern __shared__ int32_t s_hist[];                      // [num_pages] count, then (scatter) next position
   const int blocks_per_head = (a.total_q + 255) / 256;
   const int kvh = blockIdx.x / blocks_per_head;
@@ -233,6 +235,7 @@ __global__ void __launch_bounds__(1024)
 sparse_scan_kernel(const int32_t* __restrict__ bin_count, int32_t* __restrict__ bin_offset,
                    int32_t* __restrict__ bin_cursor, int4* __restrict__ items, int32_t* __restrict__ part_start,
                    int num_bins, int rows_per_item, int max_items, int tpc, int bins_per_head) {
+  chain_begin();
   __shared__ int s_ent[1024], s_itm[1024];
   __shared__ int carry_ent, carry_itm;
   if (threadIdx.x == 0) { carry_ent = 0; carry_itm = 0; }
@@ -293,6 +296,7 @@ __global__ void __launch_bounds__(MergeCfg<KBN>::WARPS * 32, 1)
 sparse_merge_kernel(const __nv_bfloat16* __restrict__ po, const float* __restrict__ pl, const int32_t* __restrict__ vmask,
                     __nv_bfloat16* __restrict__ out, float* __restrict__ lse_out, int kbn, int n_rows, int num_heads,
                     int g_shift, int64_t out_stride_tok, int64_t out_stride_head, float out_scale) {
+  chain_begin();
   using C = MergeCfg<KBN>;
   extern __shared__ __align__(128) unsigned char s_merge[];
   const int lane = threadIdx.x & 31, l16 = lane & 15;
@@ -390,6 +394,7 @@ sparse_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
                  const int4* __restrict__ items, const int32_t* __restrict__ part_start, const int part,
                  const int32_t* __restrict__ entries, float* __restrict__ partial_lse,
                  __nv_bfloat16* __restrict__ partial_o) {
+  chain_begin();
   // this launch covers the work items of kv head `part`, or all of them (part < 0)
   const int item_idx = (part >= 0 ? part_start[part] : 0) + static_cast<int>(blockIdx.x);
   if (item_idx >= part_start[part >= 0 ? part + 1 : p.num_kv_heads]) return;   // uniform: before any barrier / TMEM use
@@ -816,7 +821,7 @@ int launch_merge(const MsaFmhaParams& p, const Ws& w, cudaStream_t stream) {
   const int blocks = min(sms, (rows + per_cta - 1) / per_cta);
   int g_shift = 0;
   while ((p.num_kv_heads << g_shift) < p.num_qo_heads) ++g_shift;   // G divides 128
-  sparse_merge_kernel<KBN><<<blocks, C::WARPS * 32, C::SMEM, stream>>>(
+  launch_chained(sparse_merge_kernel<KBN>, blocks, C::WARPS * 32, C::SMEM, stream, 
       w.partial_o, w.partial_lse, w.vmask, static_cast<__nv_bfloat16*>(p.out), p.lse, p.kv_block_num, rows, p.num_qo_heads,
       g_shift, p.out_stride_tok, p.out_stride_head, p.out_scale);
   return cudaGetLastError() == cudaSuccess ? MSA_OK : MSA_ERR_LAUNCH;
@@ -872,18 +877,18 @@ int fmha_sparse_tc_launch(const MsaFmhaParams& p, cudaStream_t stream) {
   const unsigned n_blk_s = static_cast<unsigned>((p.total_q + 255) / 256) * p.num_kv_heads;
   auto index_pass = [&](bool scatter) {
     if (!smem_hist) {
-      if (scatter) sparse_index_kernel<true><<<n_blk, 256, 0, stream>>>(ia, w.bin_count, w.bin_cursor, w.entries, w.vmask);
-      else sparse_index_kernel<false><<<n_blk, 256, 0, stream>>>(ia, w.bin_count, w.bin_cursor, w.entries, w.vmask);
+      if (scatter) launch_chained(sparse_index_kernel<true>, n_blk, 256, 0, stream, ia, w.bin_count, w.bin_cursor, w.entries, w.vmask);
+      else launch_chained(sparse_index_kernel<false>, n_blk, 256, 0, stream, ia, w.bin_count, w.bin_cursor, w.entries, w.vmask);
     } else if (p.kv_block_num <= 16) {
-      if (scatter) sparse_index_smem_kernel<true, 16><<<n_blk_s, 256, hist_bytes, stream>>>(ia, w.bin_count, w.bin_cursor, w.entries, w.vmask);
-      else sparse_index_smem_kernel<false, 16><<<n_blk_s, 256, hist_bytes, stream>>>(ia, w.bin_count, w.bin_cursor, w.entries, w.vmask);
+      if (scatter) launch_chained(sparse_index_smem_kernel<true, 16>, n_blk_s, 256, hist_bytes, stream, ia, w.bin_count, w.bin_cursor, w.entries, w.vmask);
+      else launch_chained(sparse_index_smem_kernel<false, 16>, n_blk_s, 256, hist_bytes, stream, ia, w.bin_count, w.bin_cursor, w.entries, w.vmask);
     } else {
-      if (scatter) sparse_index_smem_kernel<true, 32><<<n_blk_s, 256, hist_bytes, stream>>>(ia, w.bin_count, w.bin_cursor, w.entries, w.vmask);
-      else sparse_index_smem_kernel<false, 32><<<n_blk_s, 256, hist_bytes, stream>>>(ia, w.bin_count, w.bin_cursor, w.entries, w.vmask);
+      if (scatter) launch_chained(sparse_index_smem_kernel<true, 32>, n_blk_s, 256, hist_bytes, stream, ia, w.bin_count, w.bin_cursor, w.entries, w.vmask);
+      else launch_chained(sparse_index_smem_kernel<false, 32>, n_blk_s, 256, hist_bytes, stream, ia, w.bin_count, w.bin_cursor, w.entries, w.vmask);
     }
   };
   index_pass(false);
-  sparse_scan_kernel<<<1, 1024, 0, stream>>>(w.bin_count, w.bin_offset, w.bin_cursor, w.items, w.part_start,
+  launch_chained(sparse_scan_kernel, 1, 1024, 0, stream, w.bin_count, w.bin_offset, w.bin_cursor, w.items, w.part_start,
                                              static_cast<int>(NB), rows_per_item, static_cast<int>(w.max_items), tpc,
                                              static_cast<int>(NP));
   index_pass(true);
@@ -931,10 +936,10 @@ int fmha_sparse_tc_launch(const MsaFmhaParams& p, cudaStream_t stream) {
     if (dev < 16) attr_done[f8][dev] = true;
   }
   if (f8)
-    sparse_tc_kernel<true><<<static_cast<unsigned>(w.max_items), NTHREADS, smem_bytes, stream>>>(
+    launch_chained(sparse_tc_kernel<true>, static_cast<unsigned>(w.max_items), NTHREADS, smem_bytes, stream, 
         p, tq, tk, tv, w.items, w.part_start, -1, w.entries, w.partial_lse, w.partial_o);
   else
-    sparse_tc_kernel<false><<<static_cast<unsigned>(w.max_items), NTHREADS, smem_bytes, stream>>>(
+    launch_chained(sparse_tc_kernel<false>, static_cast<unsigned>(w.max_items), NTHREADS, smem_bytes, stream, 
         p, tq, tk, tv, w.items, w.part_start, -1, w.entries, w.partial_lse, w.partial_o);
   if (cudaGetLastError() != cudaSuccess) return MSA_ERR_LAUNCH;
 

@@ -20,6 +20,7 @@ lse_merge_kernel(const void* __restrict__ po_, const float* __restrict__ pl, con
                  void* __restrict__ out_, float* __restrict__ lse_out, int num_splits, int total_q,
                  int num_heads, int64_t o_split_stride, int64_t l_split_stride, int64_t out_stride_tok,
                  int64_t out_stride_head, float out_scale) {
+  chain_begin();
   const int l16 = threadIdx.x & 15;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 4) + (threadIdx.x >> 4);   // t * H + h
   const int64_t rows = static_cast<int64_t>(total_q) * num_heads;
@@ -116,7 +117,7 @@ extern "C" int msa_lse_merge_ex(const void* partial_o, int32_t partial_dtype, co
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const unsigned nb = static_cast<unsigned>(blocks);
 #define MSA_MERGE_CASE(PB, OF)                                                                                       \
-  msa::lse_merge_kernel<PB, OF><<<nb, 256, 0, st>>>(partial_o, partial_lse, splits_per_row, out, lse_out, num_splits, \
+  msa::launch_chained(msa::lse_merge_kernel<PB, OF>, nb, 256, 0, st, partial_o, partial_lse, splits_per_row, out, lse_out, num_splits, \
                                                     total_q, num_heads, o_split_stride, lse_split_stride,           \
                                                     out_stride_tok, out_stride_head, out_scale)
   if (partial_dtype == MSA_DT_BF16) { if (out_dtype == MSA_DT_F32) MSA_MERGE_CASE(true, true); else MSA_MERGE_CASE(true, false); }

@@ -11,6 +11,7 @@ namespace msa {
 namespace {
 
 __global__ void __launch_bounds__(256) plan_device_kernel(const MsaPlanDeviceArgs a) {
+  chain_begin();
   __shared__ int s_total_q;
   const int G = a.pack;
   const int groups = a.num_qo_heads / G;
@@ -101,6 +102,5 @@ extern "C" int msa_plan_device(const MsaPlanDeviceArgs* a, msa_stream_t stream) 
   if (a->token_batch && !a->qo_start) return MSA_ERR_BAD_ARG;
   if (a->batch == 0) return MSA_OK;
   msa::NvtxRange range("msa_plan_device");
-  msa::plan_device_kernel<<<1, 256, 0, static_cast<cudaStream_t>(stream)>>>(*a);
-  return cudaGetLastError() == cudaSuccess ? MSA_OK : MSA_ERR_LAUNCH;
+  return msa::launch_chained(msa::plan_device_kernel, 1, 256, 0, static_cast<cudaStream_t>(stream), *a) == cudaSuccess ? MSA_OK : MSA_ERR_LAUNCH;
 }

@@ -82,6 +82,7 @@ score_stream_kernel(const __grid_constant__ MsaFmhaParams p) {
   const int h_r = p.num_qo_heads / p.num_kv_heads, G = p.pack;
   constexpr int e = F8 ? 1 : 2;
   const int64_t tok_bytes = p.k_stride_tok * e;
+  chain_begin();
 
   for (int base = 0; base < p.num_work; base += MAX_ITEMS) {
     const int n = min(MAX_ITEMS, p.num_work - base);
@@ -358,8 +359,7 @@ int score_stream_launch(const MsaFmhaParams& p, cudaStream_t stream) {
   // one CTA per SM, fewer only where there cannot be a page for each
   const int64_t most_pages = static_cast<int64_t>(p.num_work) * std::max(1, p.max_k_tiles);
   const int grid = static_cast<int>(std::min<int64_t>(nsm, most_pages));
-  kernels[v]<<<grid, NTHREADS, SMEM_BYTES, stream>>>(p);
-  return cudaGetLastError() == cudaSuccess ? MSA_OK : MSA_ERR_LAUNCH;
+  return launch_chained(kernels[v], grid, NTHREADS, SMEM_BYTES, stream, p) == cudaSuccess ? MSA_OK : MSA_ERR_LAUNCH;
 }
 
 }  // namespace msa

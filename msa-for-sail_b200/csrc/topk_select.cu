@@ -99,6 +99,7 @@ template <int TOPK, typename T, bool FORCED>
 __global__ void __launch_bounds__(512)
 topk_threshold_kernel(const T* __restrict__ scores, int32_t* __restrict__ out, int num_heads, int max_k_tiles,
                       int total_q, int nvp, int force_begin, int force_end_start, int slices) {
+  chain_begin();
   extern __shared__ uint32_t s_lists[];             // [slices][TOPK][32]: keys of the first scan, pages of the second
   __shared__ uint32_t s_threshold[32], s_count[16 * 32];
   __shared__ int s_quota[32];
@@ -225,6 +226,7 @@ template <int TOPK, typename T>
 __global__ void __launch_bounds__(256)
 topk_select_kernel(const T* __restrict__ scores, int32_t* __restrict__ out, int num_heads, int max_k_tiles,
                    int total_q, int nvp, int slices) {
+  chain_begin();
   using K = Key1;
   extern __shared__ __align__(8) unsigned char s_raw[];
   K* s_keys = reinterpret_cast<K*>(s_raw);          // [slices][32][TOPK]
@@ -330,6 +332,7 @@ template <int TOPK, int NK, typename T>
 __global__ void __launch_bounds__(256)
 topk_row_kernel(const T* __restrict__ scores, int32_t* __restrict__ out, int num_heads, int max_k_tiles, int total_q,
                 int nvp, int force_begin, int force_end_start) {
+  chain_begin();
   static_assert(TOPK <= 32, "one winner per lane");
   __shared__ uint32_t s_ord[8 * TOPK], s_page[8 * TOPK];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -383,6 +386,7 @@ topk_row_kernel(const T* __restrict__ scores, int32_t* __restrict__ out, int num
 
 template <int TOPK>
 __global__ void topk_identity_kernel(int32_t* __restrict__ out, size_t rows, int nvp) {
+  chain_begin();
   const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= rows * TOPK) return;
   const int c = static_cast<int>(i % TOPK);
@@ -395,20 +399,21 @@ int launch(const T* scores, int32_t* out, int H, int K, int T_, int nvp, int fb,
   if (rows == 0) return MSA_OK;
   if (nvp <= TOPK) {
     const size_t n = rows * TOPK;
-    topk_identity_kernel<TOPK><<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(out, rows, nvp);
+    launch_chained(topk_identity_kernel<TOPK>, static_cast<unsigned>((n + 255) / 256), 256, 0, stream, out, rows, nvp);
     return cudaGetLastError() == cudaSuccess ? MSA_OK : MSA_ERR_LAUNCH;
   }
   const int fe_start = fe <= nvp ? nvp - fe : 0;
   const bool one_word = sizeof(T) == 2 && fb == 0 && fe == 0 && nvp <= 65535;      // bf16 scores, nothing forced
-  // Decode-sized: a CTA per row, where fewer than 32 tokens would leave lanes of a thread-per-row kernel idle (32
-  // tokens x 1 head x 1 024 pages on a CTA per row: 7.4 us).
-  if ((T_ < 32 || one_word) && rows <= 2048 && nvp <= 256 * 32) {
+  // Decode-sized: a CTA per row.  From 32 tokens on a thread-per-row kernel has its lanes filled, and past the rows that
+  // are resident at a few CTAs per SM it wins (1 024 rows x 256 pages: 7.5 us against 18.5; 32 rows x 1 024 pages, one
+  // CTA there: 10 us against 7.4).
+  if ((T_ < 32 || rows <= 256 || one_word) && rows <= 2048 && nvp <= 256 * 32) {
     if (nvp <= 256 * 4)
-      topk_row_kernel<TOPK, 4, T><<<static_cast<unsigned>(rows), 256, 0, stream>>>(scores, out, H, K, T_, nvp, fb, fe_start);
+      launch_chained(topk_row_kernel<TOPK, 4, T>, static_cast<unsigned>(rows), 256, 0, stream, scores, out, H, K, T_, nvp, fb, fe_start);
     else if (nvp <= 256 * 8)
-      topk_row_kernel<TOPK, 8, T><<<static_cast<unsigned>(rows), 256, 0, stream>>>(scores, out, H, K, T_, nvp, fb, fe_start);
+      launch_chained(topk_row_kernel<TOPK, 8, T>, static_cast<unsigned>(rows), 256, 0, stream, scores, out, H, K, T_, nvp, fb, fe_start);
     else
-      topk_row_kernel<TOPK, 32, T><<<static_cast<unsigned>(rows), 256, 0, stream>>>(scores, out, H, K, T_, nvp, fb, fe_start);
+      launch_chained(topk_row_kernel<TOPK, 32, T>, static_cast<unsigned>(rows), 256, 0, stream, scores, out, H, K, T_, nvp, fb, fe_start);
     return cudaGetLastError() == cudaSuccess ? MSA_OK : MSA_ERR_LAUNCH;
   }
   const int tok_blocks = (T_ + 31) / 32;
@@ -423,11 +428,11 @@ int launch(const T* scores, int32_t* out, int H, int K, int T_, int nvp, int fb,
   if (one_word) {
     auto kern = topk_select_kernel<TOPK, T>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    kern<<<grid, 32 * slices, smem, stream>>>(scores, out, H, K, T_, nvp, slices);
+    launch_chained(kern, grid, 32 * slices, smem, stream, scores, out, H, K, T_, nvp, slices);
   } else {
     auto kern = fb > 0 || fe_start < nvp ? topk_threshold_kernel<TOPK, T, true> : topk_threshold_kernel<TOPK, T, false>;
     if (smem > 44 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    kern<<<grid, 32 * slices, smem, stream>>>(scores, out, H, K, T_, nvp, fb, fe_start, slices);
+    launch_chained(kern, grid, 32 * slices, smem, stream, scores, out, H, K, T_, nvp, fb, fe_start, slices);
   }
   return cudaGetLastError() == cudaSuccess ? MSA_OK : MSA_ERR_LAUNCH;
 }
