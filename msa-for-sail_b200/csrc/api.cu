@@ -1,5 +1,7 @@
 // C ABI front end: argument checks, kernel selection, the host-side dense planner.
 #include <algorithm>
+#include <functional>
+#include <queue>
 #include <vector>
 
 #include "common.cuh"
@@ -80,6 +82,31 @@ extern "C" int msa_fmha_fwd(const MsaFmhaParams* pp, msa_stream_t stream_) {
   return msa::fmha_mma_launch(p, stream);
 }
 
+namespace msa {
+struct Proto { int b, row0, nrows, ntiles; };      // the rows of one work item and their KV tiles, before any split
+
+// Tile times until the last of `slots` workers is done when every item is cut into pieces of `chunk` tiles and the
+// pieces are handed out longest first.  A piece costs three tiles beyond its own (a CTA's dependent index loads, the
+// latency of its first tile, its epilogue).
+static int makespan(const std::vector<Proto>& protos, int groups, int chunk, int slots) {
+  constexpr int kPieceCost = 3;
+  std::vector<int> pieces;
+  for (const Proto& pr : protos)
+    for (int t = pr.ntiles; t > 0; t -= chunk) pieces.push_back(std::min(t, chunk) + kPieceCost);
+  std::sort(pieces.begin(), pieces.end(), std::greater<int>());
+  std::priority_queue<int, std::vector<int>, std::greater<int>> load(std::greater<int>(), std::vector<int>(slots, 0));
+  int last = 0;
+  for (const int t : pieces)
+    for (int g = 0; g < groups; ++g) {
+      const int end = load.top() + t;
+      load.pop();
+      load.push(end);
+      last = std::max(last, end);
+    }
+  return last;
+}
+}  // namespace msa
+
 extern "C" int msa_plan_dense(const MsaPlanArgs* a, MsaWorkItem* work, int32_t capacity, int32_t* splits_per_row,
                               int32_t* max_splits_out) {
   if (!a || !a->qo_len || !a->kv_len || !a->qo_offset || (!work && capacity > 0)) return MSA_ERR_BAD_ARG;
@@ -91,7 +118,7 @@ extern "C" int msa_plan_dense(const MsaPlanArgs* a, MsaWorkItem* work, int32_t c
   const int groups = a->num_qo_heads / G;
   const int bm_eff = (a->block_m / G) * G;       // a token's heads never straddle two items
 
-  struct Proto { int b, row0, nrows, ntiles; };
+  using msa::Proto;
   std::vector<Proto> protos;
   int max_tiles = 0;
   for (int b = 0; b < a->batch; ++b) {
@@ -120,6 +147,17 @@ extern "C" int msa_plan_dense(const MsaPlanArgs* a, MsaWorkItem* work, int32_t c
       int want = static_cast<int>((2LL * sms + items - 1) / items);
       want = std::min(want, ceiling);
       chunk = std::max(4, (max_tiles + want - 1) / want);      // at least 512 keys per split
+    }
+    // Decode: one row tile per batch item.  Cutting the items at just above the average load of an SM gives nearly every
+    // SM one full piece and leaves the remainders to fill up the rest; whichever of the two cuts ends earlier is taken.
+    // (Ragged lengths are where it pays: 31 sequences of 515 to 7 001 keys x 4 heads: 28 tile times against 40.)
+    if (max_tiles > 4 && static_cast<int>(protos.size()) <= a->batch && items < 8LL * sms) {
+      const int slots = sms * std::max(1, a->ctas_per_sm);
+      long long total = 0;
+      for (const Proto& pr : protos) total += static_cast<long long>(pr.ntiles) * groups;
+      int cut = std::max(4, static_cast<int>((total * 103 + 100LL * slots - 1) / (100LL * slots)));
+      cut = std::max(cut, (max_tiles + ceiling - 1) / ceiling);
+      if (cut < max_tiles && msa::makespan(protos, groups, cut, slots) < msa::makespan(protos, groups, chunk, slots)) chunk = cut;
     }
   }
   std::vector<MsaWorkItem> items;

@@ -54,7 +54,7 @@ class MsaFmhaParams(ctypes.Structure):
 class MsaPlanArgs(ctypes.Structure):
     _fields_ = [("qo_len", _p), ("kv_len", _p), ("qo_offset", _p), ("batch", _i32),
                 ("num_qo_heads", _i32), ("num_kv_heads", _i32), ("block_m", _i32), ("pack", _i32),
-                ("num_splits", _i32), ("num_sms", _i32), ("reserved", _i32)]
+                ("num_splits", _i32), ("num_sms", _i32), ("ctas_per_sm", _i32)]
 
 
 class MsaPlanDeviceArgs(ctypes.Structure):

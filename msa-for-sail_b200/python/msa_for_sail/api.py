@@ -360,7 +360,8 @@ def _fmha_sail_plan(
         info["token_batch"] = None
         args = _lib.MsaPlanArgs(
             a_q.ctypes.data, a_k.ctypes.data, a_o.ctypes.data, batch, num_qo_heads, hkv, block_m, pack,
-            num_kv_splits if num_kv_splits >= 1 else -128, num_sms, 0)
+            num_kv_splits if num_kv_splits >= 1 else -128, num_sms,
+            2 if use_fp8_kvcache and max_qo * pack <= 16 else 1)      # two CTAs of the e4m3 decode kernel share an SM
         cap = 1024
         spr = np.ones(max(1, total_q), np.int32)
         max_splits = _lib._i32(1)

@@ -114,6 +114,47 @@ def test_planner_reports_capacity():
     assert L.lib.msa_plan_dense(ctypes.byref(args), work.ctypes.data, 2, None, None) == -4
 
 
+@pytest.mark.parametrize("seed", range(8))
+@pytest.mark.parametrize("ctas", [1, 2])
+def test_host_planner_cuts_ragged_decode_evenly(seed, ctas):
+    """Adaptive splits of ragged decode lengths: every tile once, and the longest-first schedule of the pieces ends no
+    later than that of the plain rule (pieces for two waves of the SMs)."""
+    import heapq
+    L = _lib()
+    rng = np.random.default_rng(seed)
+    kv = rng.integers(1, [600, 5000, 40000, 200000][seed % 4], int(rng.integers(1, 60))).tolist()
+    hk = [1, 2, 4, 8][seed % 4]
+    one = np.ones(len(kv), np.int32)
+    a_k = np.asarray(kv, np.int32)
+    off = a_k - 1
+    args = L.MsaPlanArgs(one.ctypes.data, a_k.ctypes.data, off.ctypes.data, len(kv), hk * 8, hk, 16, 8, -128, 148, ctas)
+    work = np.empty((20000, 8), np.int32)
+    spr, most = np.zeros(len(kv), np.int32), ctypes.c_int32(0)
+    n = L.lib.msa_plan_dense(ctypes.byref(args), work.ctypes.data, 20000, spr.ctypes.data, ctypes.byref(most))
+    assert n > 0
+    pieces = {}
+    for b, h0, r0, tb, te, sp, nr, _ in work[:n].tolist():
+        pieces.setdefault((b, h0), []).append((sp, tb, te))
+    assert len(pieces) == len(kv) * hk
+    for (b, _), v in pieces.items():
+        v.sort()
+        assert [x[0] for x in v] == list(range(spr[b])) and spr[b] <= most.value <= 128
+        assert v[0][1] == 0 and v[-1][2] == -(-kv[b] // 128)
+        assert all(x[2] == y[1] for x, y in zip(v, v[1:]))
+
+    def ends(sizes):
+        load = [0] * (148 * ctas)
+        for t in sorted(sizes, reverse=True):
+            heapq.heappush(load, heapq.heappop(load) + t + 3)
+        return max(load)
+
+    tiles = [-(-x // 128) for x in kv]
+    items = len(kv) * hk
+    plain = max(tiles) if items >= 296 else max(4, -(-max(tiles) // -(-296 // items)))
+    plain_sizes = [min(x, s + plain) - s for x in tiles for s in range(0, x, plain) for _ in range(hk)]
+    assert ends((work[:n, 4] - work[:n, 3]).tolist()) <= ends(plain_sizes)
+
+
 def test_api_surface_matches_upstream_names():
     import inspect
     import msa_for_sail as m
