@@ -115,6 +115,22 @@ def _compute_pack_factor(max_qo_len, num_qo_heads, num_kv_heads):
     return h_r
 
 
+def _sparse_splits(items, kv_block_num, most, num_sms, two_per_sm):
+    """Splits of the selected pages in token-major sparse attention: `most`, halved as often as pays.  A CTA takes its
+    pages and about four page times more (dependent index loads, the first page's latency, the epilogue), the CTAs run in
+    rounds of the slots there are (two e4m3 CTAs of at most 16 rows share an SM), and splits cost a merge, about four
+    page times.  24 tokens x 4 heads x 16 bf16 pages: 192 CTAs of 8 pages and the merge 36 us, 96 of 16 pages 26 us."""
+    slots = num_sms * (2 if two_per_sm else 1)
+    best, best_cost = 1, None
+    s = min(most, kv_block_num)
+    while s >= 1:
+        cost = -(-items * s // slots) * (-(-kv_block_num // s) + 4) + (4 if s > 1 else 0)
+        if best_cost is None or cost <= best_cost:
+            best, best_cost = s, cost
+        s //= 2
+    return best
+
+
 def _block_m(rows):
     return 16 if rows <= 16 else (64 if rows <= 64 else 128)
 
@@ -337,18 +353,8 @@ def _fmha_sail_plan(
     num_work = 0
     info["work"] = info["num_kv_splits_per_row"] = None
     if is_sparse:
-        items = total_q * hkv
-        if num_kv_splits >= 1:
-            # an explicit count is an upper bound: once the (token, KV head) items alone give every
-            # SM a CTA, further splitting only adds per-CTA prologue/epilogue latency and a merge
-            # pass (the result does not depend on the split count)
-            splits = min(num_kv_splits, kv_block_num)
-            while splits > 1 and items * (splits // 2) >= num_sms:
-                splits //= 2
-        else:
-            splits = 1
-            while splits * 2 <= min(kv_block_num, 8) and items * splits < 2 * num_sms:
-                splits *= 2
+        splits = _sparse_splits(total_q * hkv, kv_block_num, num_kv_splits if num_kv_splits >= 1 else 8, num_sms,
+                                use_fp8_kvcache and h_r <= 16)
         up.add("token_batch", np.repeat(np.arange(batch, dtype=np.int32), a_q))
         up.add("page_batch", np.repeat(np.arange(batch, dtype=np.int32), pages_per))
         info["num_logical_pages"] = int(pages_per.sum())
@@ -457,12 +463,11 @@ def _fmha_sail_plan_device(qo_segment_lens, kv_segment_lens, num_qo_heads, hkv, 
     is_sparse = kv_block_num > 0 and page_size > 0
     if is_sparse:
         pack, block_m = h_r, _block_m(h_r)
-        splits = min(num_kv_splits, kv_block_num) if num_kv_splits >= 1 else 1
         num_sms = _num_sms(dev)
         if usable_SM_count > 0:
             num_sms = min(num_sms, usable_SM_count)
-        while splits > 1 and max_total_q * hkv * (splits // 2) >= num_sms:
-            splits //= 2
+        splits = _sparse_splits(max_total_q * hkv, kv_block_num, max(1, num_kv_splits), num_sms,
+                                use_fp8_kvcache and h_r <= 16)
     else:
         pack = _compute_pack_factor(max_qo, num_qo_heads, hkv)
         block_m = _block_m(max_qo * pack)
