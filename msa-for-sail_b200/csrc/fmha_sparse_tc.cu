@@ -74,7 +74,11 @@ constexpr int REGS_NEEDED = NWG * 128 * REGS_SOFTMAX + (GATHER_WARPS + 1) * 32 *
 static_assert(NTHREADS == (MMA_WARP + 1) * 32, "warp roles");
 static_assert(REGS_NEEDED <= 65536, "setmaxnreg budget");
 constexpr int ITEM_CHUNKS = 32;                 // chunks of 128 rows per work item
-constexpr uint32_t kEmuMask = 0x5252;
+// Pairs (of 16 per 32 columns) whose exp2 runs on the FMA pipe.  At 2 x 32 768 tokens in bf16 a whole pass takes 10.6 ms
+// with none, 10.2 ms with two of 16 and 9.9 ms with six; in e4m3, whose conversions fill the ALU already, none is best
+// (1 616 us against 1 635 us with two and about 1 660 us with six for a chunk of 8 192 tokens).
+template <bool F8>
+constexpr uint32_t kEmuMask = F8 ? 0x0000 : 0x5252;
 
 // TMEM: three S buffers (P_c overwrites the front of S_c) and one O.  Q_{c+3} K^T reuses the buffer of
 // chunk c, so it follows P_c V directly in the MMA warp's program and is ready long before its
@@ -709,7 +713,7 @@ sparse_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
           const uint64_t x2 = f2_fma(f2_pack(__uint_as_float(sv[cc][e]), __uint_as_float(sv[cc][e + 1])), scale2, negm2);
           float p0, p1, x0, x1;
           f2_unpack(x2, x0, x1);
-          if ((kEmuMask >> ((e >> 1) & 15)) & 1) {
+          if ((kEmuMask<F8> >> ((e >> 1) & 15)) & 1) {
             const uint64_t xc = f2_pack(fmaxf(x0, -126.f), fmaxf(x1, -126.f));
             const uint64_t t2 = f2_add(xc, f2_pack(12582912.f, 12582912.f));
             const uint64_t n2 = f2_add(t2, f2_pack(-12582912.f, -12582912.f));
