@@ -73,7 +73,10 @@ constexpr int REGS_SOFTMAX = 152, REGS_OTHER = 40;
 constexpr int REGS_NEEDED = NWG * 128 * REGS_SOFTMAX + (GATHER_WARPS + 1) * 32 * REGS_OTHER;
 static_assert(NTHREADS == (MMA_WARP + 1) * 32, "warp roles");
 static_assert(REGS_NEEDED <= 65536, "setmaxnreg budget");
-constexpr int ITEM_CHUNKS = 32;                 // chunks of 128 rows per work item
+// Chunks of 128 rows per work item: a list of one page in pieces of 32, of 16 where an SM gets fewer than 128 chunks in
+// all and the last round weighs more than the pages loaded twice (9 000 tokens x 16 heads x 8 pages: 193 us a pass
+// against 198; 8: 205.  65 536 chunks: 1 654 us with 16, 1 620 with 32; 524 288 chunks: 32, 64 and 128 within 1 %).
+inline int item_chunks(int64_t rows) { return rows < int64_t(148) * 128 * BM ? 16 : 32; }
 // Pairs (of 16 per 32 columns) whose exp2 runs on the FMA pipe.  At 2 x 32 768 tokens in bf16 a whole pass takes 10.6 ms
 // with none, 10.2 ms with two of 16 and 9.9 ms with six; in e4m3, whose conversions fill the ALU already, none is best
 // (1 616 us against 1 635 us with two and about 1 660 us with six for a chunk of 8 192 tokens).
@@ -119,7 +122,7 @@ Ws carve(void* base, int64_t T, int Hq, int Hkv, int kbn, int64_t NP) {
   const int G = Hq / Hkv;
   const int64_t tpc = BM / G;
   w.cap = T * Hkv * kbn + NB * tpc;
-  w.max_items = (T * Hkv * kbn) / (tpc * ITEM_CHUNKS) + NB + 1;
+  w.max_items = (T * Hkv * kbn) / (tpc * item_chunks(T * Hq * kbn)) + NB + 1;
   char* p = static_cast<char*>(base);
   int64_t off = 0;
   auto take = [&](int64_t bytes) { char* r = p ? p + off : nullptr; off = align256(off + bytes); return r; };
@@ -234,32 +237,40 @@ sparse_index_smem_kernel(const IndexArgs a, int32_t* __restrict__ bin_count, int
   }
 }
 
-// exclusive scan of the bin counts + work items (one CTA; NB is a few thousand to ~1e5)
+// exclusive scan of the bin counts + work items (one CTA; NB is a few thousand to ~1e5).  Warp scans and two barriers
+// per 1 024 bins; a scan in shared memory with a barrier pair per step made twenty-two (193 against 192 us a pass at 9 000
+// tokens, 1 620 against 1 593 us at 3 076 bins).
 __global__ void __launch_bounds__(1024)
 sparse_scan_kernel(const int32_t* __restrict__ bin_count, int32_t* __restrict__ bin_offset,
                    int32_t* __restrict__ bin_cursor, int4* __restrict__ items, int32_t* __restrict__ part_start,
                    int num_bins, int rows_per_item, int max_items, int tpc, int bins_per_head) {
   chain_begin();
-  __shared__ int s_ent[1024], s_itm[1024];
-  __shared__ int carry_ent, carry_itm;
-  if (threadIdx.x == 0) { carry_ent = 0; carry_itm = 0; }
-  __syncthreads();
+  __shared__ int s_ent[32], s_itm[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int carry_ent = 0, carry_itm = 0;
   for (int base = 0; base < num_bins; base += 1024) {
     const int bin = base + threadIdx.x;
     const int cnt = bin < num_bins ? bin_count[bin] : 0;
     const int cnt_pad = (cnt + tpc - 1) / tpc * tpc;        // a bin starts on a chunk boundary
     const int nit = (cnt + rows_per_item - 1) / rows_per_item;
-    s_ent[threadIdx.x] = cnt_pad; s_itm[threadIdx.x] = nit;
+    // inclusive scan in the warp, then over the sums of the 32 warps (each warp does that for itself)
+    auto scan = [&](int v) {
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, v, d);
+        if (lane >= d) v += o;
+      }
+      return v;
+    };
+    const int ent = scan(cnt_pad), itm = scan(nit);
+    if (lane == 31) { s_ent[warp] = ent; s_itm[warp] = itm; }
     __syncthreads();
-    for (int d = 1; d < 1024; d <<= 1) {                   // Hillis-Steele inclusive scan
-      const int e = threadIdx.x >= d ? s_ent[threadIdx.x - d] : 0;
-      const int i2 = threadIdx.x >= d ? s_itm[threadIdx.x - d] : 0;
-      __syncthreads();
-      s_ent[threadIdx.x] += e; s_itm[threadIdx.x] += i2;
-      __syncthreads();
-    }
-    const int ent0 = carry_ent + s_ent[threadIdx.x] - cnt_pad;
-    const int itm0 = carry_itm + s_itm[threadIdx.x] - nit;
+    const int warp_ent = scan(s_ent[lane]), warp_itm = scan(s_itm[lane]);
+    const int before_ent = __shfl_sync(0xffffffffu, warp_ent, max(0, warp - 1)), before_itm = __shfl_sync(0xffffffffu, warp_itm, max(0, warp - 1));
+    const int ent0 = carry_ent + (warp > 0 ? before_ent : 0) + ent - cnt_pad;
+    const int itm0 = carry_itm + (warp > 0 ? before_itm : 0) + itm - nit;
+    carry_ent += __shfl_sync(0xffffffffu, warp_ent, 31);
+    carry_itm += __shfl_sync(0xffffffffu, warp_itm, 31);
     if (bin < num_bins) {
       if (bin % bins_per_head == 0) part_start[bin / bins_per_head] = min(itm0, max_items);
       bin_offset[bin] = ent0;
@@ -268,8 +279,6 @@ sparse_scan_kernel(const int32_t* __restrict__ bin_count, int32_t* __restrict__ 
         if (itm0 + k < max_items)
           items[itm0 + k] = make_int4(bin, ent0 + k * rows_per_item, min(ent0 + cnt, ent0 + (k + 1) * rows_per_item), 0);
     }
-    __syncthreads();
-    if (threadIdx.x == 1023) { carry_ent += s_ent[1023]; carry_itm += s_itm[1023]; }
     __syncthreads();
   }
   if (threadIdx.x == 0) { bin_offset[num_bins] = carry_ent; part_start[num_bins / bins_per_head] = min(carry_itm, max_items); }
@@ -875,7 +884,7 @@ int fmha_sparse_tc_launch(const MsaFmhaParams& p, cudaStream_t stream) {
   const int64_t n_thr = static_cast<int64_t>(p.total_q) * p.num_kv_heads;
   const unsigned n_blk = static_cast<unsigned>((n_thr + 255) / 256);
   const int tpc = BM / G;
-  const int rows_per_item = tpc * ITEM_CHUNKS;
+  const int rows_per_item = tpc * item_chunks(static_cast<int64_t>(p.total_q) * p.num_qo_heads * p.kv_block_num);
   const size_t hist_bytes = static_cast<size_t>(NP) * 4;
   const bool smem_hist = hist_bytes <= 48 * 1024;
   const unsigned n_blk_s = static_cast<unsigned>((p.total_q + 255) / 256) * p.num_kv_heads;
