@@ -156,7 +156,14 @@ extern "C" int msa_plan_dense(const MsaPlanArgs* a, MsaWorkItem* work, int32_t c
       long long total = 0;
       for (const Proto& pr : protos) total += static_cast<long long>(pr.ntiles) * groups;
       int cut = std::max(4, static_cast<int>((total * 103 + 100LL * slots - 1) / (100LL * slots)));
-      cut = std::max(cut, (max_tiles + ceiling - 1) / ceiling);
+      // no more splits than the ceiling, nor than the library's own scratch holds where the plain cut fits it
+      long long rows = 0;
+      for (int b = 0; b < a->batch; ++b) rows += static_cast<long long>(a->qo_len[b]) * a->num_qo_heads;
+      const int plain_splits = (max_tiles + chunk - 1) / chunk;
+      int most = ceiling;
+      if (plain_splits * rows <= MSA_STATIC_SCRATCH_MAX_ROWS)
+        most = static_cast<int>(std::min<long long>(most, MSA_STATIC_SCRATCH_MAX_ROWS / std::max(1LL, rows)));
+      cut = std::max(cut, (max_tiles + most - 1) / most);
       if (cut < max_tiles && msa::makespan(protos, groups, cut, slots) < msa::makespan(protos, groups, chunk, slots)) chunk = cut;
     }
   }

@@ -132,6 +132,10 @@ def test_host_planner_cuts_ragged_decode_evenly(seed, ctas):
     spr, most = np.zeros(len(kv), np.int32), ctypes.c_int32(0)
     n = L.lib.msa_plan_dense(ctypes.byref(args), work.ctypes.data, 20000, spr.ctypes.data, ctypes.byref(most))
     assert n > 0
+    tiles = [-(-x // 128) for x in kv]
+    items = len(kv) * hk
+    plain = max(tiles) if items >= 296 else max(4, -(-max(tiles) // -(-296 // items)))
+    plain_splits, rows = -(-max(tiles) // plain), len(kv) * hk * 8
     pieces = {}
     for b, h0, r0, tb, te, sp, nr, _ in work[:n].tolist():
         pieces.setdefault((b, h0), []).append((sp, tb, te))
@@ -139,6 +143,8 @@ def test_host_planner_cuts_ragged_decode_evenly(seed, ctas):
     for (b, _), v in pieces.items():
         v.sort()
         assert [x[0] for x in v] == list(range(spr[b])) and spr[b] <= most.value <= 128
+        if plain_splits * rows <= 16384:                     # what fits the library's own scratch goes on fitting it
+            assert most.value * rows <= 16384
         assert v[0][1] == 0 and v[-1][2] == -(-kv[b] // 128)
         assert all(x[2] == y[1] for x, y in zip(v, v[1:]))
 
@@ -148,9 +154,6 @@ def test_host_planner_cuts_ragged_decode_evenly(seed, ctas):
             heapq.heappush(load, heapq.heappop(load) + t + 3)
         return max(load)
 
-    tiles = [-(-x // 128) for x in kv]
-    items = len(kv) * hk
-    plain = max(tiles) if items >= 296 else max(4, -(-max(tiles) // -(-296 // items)))
     plain_sizes = [min(x, s + plain) - s for x in tiles for s in range(0, x, plain) for _ in range(hk)]
     assert ends((work[:n, 4] - work[:n, 3]).tolist()) <= ends(plain_sizes)
 
