@@ -24,7 +24,7 @@
 //
 // TMEM (512 columns): S_A [0,128) S_B [128,256) O_A [256,384) O_B [384,512); P aliases the
 // first 64 columns of its S (32 in e4m3).  Shared memory: Q 64 KB, K 2x32 KB, V 2x32 KB (e4m3:
-// Q 32 KB, K 4x16 KB, V 4x16 KB), all in the 128-byte-swizzled layout that both TMA and the UMMA
+// Q 32 KB, K 4x16 KB, V 4x16 KB; score-only: K 2x64 KB or 4x32 KB in the same space), all in the 128-byte-swizzled layout that both TMA and the UMMA
 // descriptors understand.
 //
 // A CTA takes one work item after the other (see the scheduler), so that the loads and the first S of an
@@ -104,6 +104,12 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
   using C = Cfg<F8>;
   constexpr int TILE_BYTES = C::TILE_BYTES, NSUB = C::NSUB, SUB_ELEMS = C::SUB_ELEMS;
   constexpr int KSTAGES = C::STAGES, VSTAGES = C::STAGES;
+  // Score-only pass: K comes in pairs of tiles (256 keys, one MMA of N = 256 per K step) through the space of both rings:
+  // two pairs in bf16, four in e4m3; S of a Q tile is 256 columns of TMEM.  With N = 128 an MMA reads as much of Q as of K
+  // from shared memory and, with nothing else to hide that, took 125 clocks instead of 64.  65 536 rows x 16 384 keys on
+  // average, bf16: 250 -> 207 us; 8 192 rows x 4 heads x 94 000 keys, e4m3: 431 -> 350 us.
+  constexpr int PAIR_BYTES = 2 * TILE_BYTES;
+  static_assert(HAS_O || KSTAGES * PAIR_BYTES <= C::OFF_BAR - C::OFF_K, "pairs of K tiles fit both rings");
   constexpr int OFF_Q = C::OFF_Q, OFF_K = C::OFF_K, OFF_V = C::OFF_V, OFF_BAR = C::OFF_BAR;
   constexpr float kRescaleThreshold = C::kRescaleThreshold, kPOffset = C::kPOffset;
   extern __shared__ unsigned char smem_raw[];
@@ -210,7 +216,35 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
     } else if (lane == 0) {
       mbar_arrive(bar(NEXT_REQ));
     }
-    for (int j = 0; j < n_total && alive; ++j, ++tile) {
+    if constexpr (!HAS_O) {
+      for (int j = 0; j < n_total; j += 2, ++tile) {
+        if (stall_tile >= 0 && j >= stall_tile) { alive = false; break; }
+        if (j / 2 == max(0, n_total - NEXT_LEAD) / 2 && lane == 0) mbar_arrive(bar(NEXT_REQ));
+        const int ks = tile % KSTAGES, tiles = min(2, n_total - j);
+        int page[2] = {0, 0};
+        if (paged) {
+          page[0] = chk(p.kv_indices[page_base + j], 0, static_cast<int>(p.kv_extent), p.status);
+          if (tiles == 2) page[1] = chk(p.kv_indices[page_base + j + 1], 0, static_cast<int>(p.kv_extent), p.status);
+        }
+        alive = __all_sync(0xffffffffu, mbar_wait(bar(K_EMPTY + ks), ((tile / KSTAGES) & 1) ^ 1, abort_flag, spin_limit));
+        if (!alive) break;
+        if (elect_one()) {
+          mbar_arrive_expect_tx(bar(K_FULL + ks), tiles * TILE_BYTES);
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            if (t >= tiles) break;
+#pragma unroll
+            for (int hlf = 0; hlf < NSUB; ++hlf) {       // a half of head_dim: 256 rows of 128 bytes
+              const uint32_t dst = smem_base + OFF_K + ks * PAIR_BYTES + (2 * hlf + t) * SUB_BYTES;
+              if (paged) tma_load_4d(dst, &tm_k, bar(K_FULL + ks), hlf * SUB_ELEMS, 0, kvh, page[t]);
+              else tma_load_3d(dst, &tm_k, bar(K_FULL + ks), hlf * SUB_ELEMS, kvh, kv_base + (j + t) * BN);
+            }
+          }
+        }
+        __syncwarp();
+      }
+    } else
+      for (int j = 0; j < n_total && alive; ++j, ++tile) {
       if (j == stall_tile) { alive = false; break; }    // test hook: whoever waits for this tile runs out of polls
       if (j == max(0, n_total - NEXT_LEAD) && lane == 0) mbar_arrive(bar(NEXT_REQ));
       const int ks = tile % KSTAGES, vs = tile % VSTAGES;
@@ -231,7 +265,6 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
         }
       }
       __syncwarp();
-      if (!has_o) continue;
       alive = mbar_wait(bar(V_EMPTY + vs), ((tile / VSTAGES) & 1) ^ 1, abort_flag, spin_limit);
       if (lane == 0) trace(3, j, 2);
       if (!alive) break;
@@ -246,7 +279,7 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
         }
       }
       __syncwarp();
-      if (fix && alive && has_o) {
+      if (fix && alive) {
         alive = mbar_wait(bar(V_FIX), fix_phase, abort_flag, spin_limit);
         alive = __all_sync(0xffffffffu, alive);
         fix_phase ^= 1;
@@ -356,7 +389,8 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
       }
     };
     uint32_t tile = 0, q_loads = 0;                    // running counts, as in the producer
-    uint32_t p_par = 0;                                // bit x: parity of the next P_FULL + x
+    [[maybe_unused]] uint32_t p_par = 0;               // bit x: parity of the next P_FULL + x
+    [[maybe_unused]] uint32_t n_s[2] = {0, 0};         // score-only: S pairs issued so far
     bool alive = true;
     Item w;
     for (uint32_t it = 0; take_item(it, w, alive); ++it) {
@@ -364,6 +398,41 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
       if (n_total == 0) continue;
       alive = mbar_wait(bar(Q_FULL), q_loads & 1, abort_flag, spin_limit);
       ++q_loads;
+      if constexpr (!HAS_O) {
+        constexpr uint32_t IDESC_PAIR = F8 ? idesc_e4m3(BM, 2 * BN, false, false) : idesc_bf16(BM, 2 * BN, false, false);
+        for (int j = 0; j < n_total && alive; j += 2, ++tile) {
+          alive = mbar_wait(bar(K_FULL + tile % KSTAGES), (tile / KSTAGES) & 1, abort_flag, spin_limit);
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            if (j >= w.n_tiles[x] || !alive) continue;
+            const uint32_t u = n_s[x]++;
+            if (u > 0) alive = mbar_wait(bar(P_FULL + x), (u - 1) & 1, abort_flag, spin_limit);   // S has been read
+            alive = __all_sync(0xffffffffu, alive);
+            if (!alive) break;
+            tc_fence_after();
+            if (elect_one()) {
+              const uint32_t qa = (smem_base + OFF_Q + x * TILE_BYTES) >> 4;
+              const uint32_t ka = (smem_base + OFF_K + (tile % KSTAGES) * PAIR_BYTES) >> 4;
+#pragma unroll
+              for (int k = 0; k < KSTEPS; ++k) {
+                const uint32_t oq = ((k >> 2) * SUB_BYTES + (k & 3) * 32) >> 4, ok = ((k >> 2) * 2 * SUB_BYTES + (k & 3) * 32) >> 4;
+                if constexpr (F8) mma_ss_f8(tmem + x * 2 * BN, dk_hi | ((qa + oq) & 0x3FFF), dk_hi | ((ka + ok) & 0x3FFF), IDESC_PAIR, k > 0);
+                else mma_ss(tmem + x * 2 * BN, dk_hi | ((qa + oq) & 0x3FFF), dk_hi | ((ka + ok) & 0x3FFF), IDESC_PAIR, k > 0);
+              }
+              mma_commit(bar(S_FULL + x));
+            }
+            __syncwarp();
+          }
+          alive = __all_sync(0xffffffffu, alive);
+          if (!alive) break;
+          if (elect_one()) {
+            mma_commit(bar(K_EMPTY + tile % KSTAGES));
+            if (j + 2 >= n_total) mma_commit(bar(Q_EMPTY));
+          }
+          __syncwarp();
+        }
+        continue;
+      }
       if (alive) alive = mbar_wait(bar(K_FULL + tile % KSTAGES), (tile / KSTAGES) & 1, abort_flag, spin_limit);
       alive = __all_sync(0xffffffffu, alive);
       if (!alive) break;
@@ -384,7 +453,7 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
           const bool more = j + 1 < w.n_tiles[x];
           // the tiles this step reads normally landed long ago: check them before P, and only once per j
           if (x == 0 || j >= w.n_tiles[0]) {
-            if (has_o) alive = mbar_wait(bar(V_FULL + tile % VSTAGES), (tile / VSTAGES) & 1, abort_flag, spin_limit);
+            alive = mbar_wait(bar(V_FULL + tile % VSTAGES), (tile / VSTAGES) & 1, abort_flag, spin_limit);
             if (alive && j + 1 < n_total)
               alive = mbar_wait(bar(K_FULL + (tile + 1) % KSTAGES), ((tile + 1) / KSTAGES) & 1, abort_flag, spin_limit);
           }
@@ -395,15 +464,15 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
           tc_fence_after();
           if (lane == 0) trace(2, j, x * 4 + 2);
           if (elect_one()) {
-            if (has_o) issue_pv(x, tile, j == 0);
+            issue_pv(x, tile, j == 0);
             if (more) {
               issue_qk(x, tile + 1);
               mma_commit(bar(S_FULL + x));
-            } else if (has_o) {
+            } else {
               mma_commit(bar(O_FULL + x));
             }
             if (x == 1 || j >= w.n_tiles[1]) {          // last user of this V stage / next K stage
-              if (has_o) mma_commit(bar(V_EMPTY + tile % VSTAGES));
+              mma_commit(bar(V_EMPTY + tile % VSTAGES));
               if (j + 1 < n_total) mma_commit(bar(K_EMPTY + (tile + 1) % KSTAGES));
               if (j + 2 == n_total) mma_commit(bar(Q_EMPTY));   // the last Q K^T of the item has been issued
             }
@@ -421,7 +490,6 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
     const int x = warp >> 2;                             // 0: tile A, 1: tile B
     const int r = ((warp & 3) << 5) | lane;              // row in tile == TMEM lane
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) << 5) << 16;
-    const uint32_t tS = tmem + x * BN + lane_addr;
     const uint32_t tO = tmem + 256 + x * kHeadDim + lane_addr;
     const bool want_score = (p.flags & MSA_FLAG_OUT_SCORE) != 0 && p.max_score != nullptr;
     bool alive = true;
@@ -441,9 +509,12 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
 
     for (int j = 0; j < nx && alive; ++j) {
       if (r == 0) trace(x, j, 0);
-      alive = __all_sync(0xffffffffu, mbar_wait(bar(S_FULL + x), s_par, abort_flag, spin_limit));
-      if (!alive) break;                                 // the warp votes below: all of it goes on, or none
-      s_par ^= 1;
+      if (HAS_O || (j & 1) == 0) {                       // score-only: S of two tiles at a time
+        alive = __all_sync(0xffffffffu, mbar_wait(bar(S_FULL + x), s_par, abort_flag, spin_limit));
+        if (!alive) break;                               // the warp votes below: all of it goes on, or none
+        s_par ^= 1;
+      }
+      const uint32_t tS = tmem + (HAS_O ? x * BN : x * 2 * BN + (j & 1) * BN) + lane_addr;
       tc_fence_after();
       if (r == 0) trace(x, j, 1);
       const int pos0 = j * BN;
@@ -456,6 +527,10 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
       tmem_ld32(tS + 96, sv[3]);
       tmem_wait_ld();
       if (r == 0) trace(x, j, 2);
+      if (!HAS_O && ((j & 1) || j + 1 == nx)) {          // both tiles' S are out: it may be filled again
+        tc_fence_before();
+        mbar_arrive(bar(P_FULL + x));
+      }
       if (need_mask) {
 #pragma unroll
         for (int c = 0; c < 4; ++c)
@@ -470,7 +545,7 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
           else static_cast<float*>(p.max_score)[o] = mx;
         }
       };
-      if (!has_o) {                    // score-only pass: the row max of the tile, then S goes back to the MMA warp
+      if (!has_o) {                    // score-only pass: the row max of the tile
         float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};        // four independent chains
 #pragma unroll
         for (int c = 0; c < 4; ++c)
@@ -478,8 +553,6 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
           for (int e = 0; e < 32; e += 2)
             m4[(e >> 1) & 3] = max3(m4[(e >> 1) & 3], __uint_as_float(sv[c][e]), __uint_as_float(sv[c][e + 1]));
         store_score(fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])));
-        tc_fence_before();
-        mbar_arrive(bar(P_FULL + x));
         continue;
       }
       // P = exp2(S * scale - m) as bf16 / e4m3, written over the front of S; the row max of the tile (the
