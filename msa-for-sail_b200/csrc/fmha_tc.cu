@@ -197,105 +197,106 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
     bool alive = true;
     Item w;
     for (uint32_t it = 0; take_item(it, w, alive); ++it) {
-    const int n_total = max(w.n_tiles[0], w.n_tiles[1]), head = w.head, kvh = w.kvh, kv_len = w.kv_len;
-    const int page_base = w.kv0, kv_base = w.kv0;
-    if (n_total > 0) {                                  // an item without visible keys loads nothing
-      alive = __all_sync(0xffffffffu, mbar_wait(bar(Q_EMPTY), (q_loads & 1) ^ 1, abort_flag, spin_limit));
-      if (!alive) break;
-      ++q_loads;
-      if (elect_one()) {
-        mbar_arrive_expect_tx(bar(Q_FULL), 2 * TILE_BYTES);
-#pragma unroll
-        for (int x = 0; x < 2; ++x)
-#pragma unroll
-          for (int hlf = 0; hlf < NSUB; ++hlf)
-            tma_load_3d(smem_base + OFF_Q + x * TILE_BYTES + hlf * SUB_BYTES, &tm_q, bar(Q_FULL), hlf * SUB_ELEMS, head,
-                        w.qo_base + w.row0 + x * BM);
-      }
-      __syncwarp();
-    } else if (lane == 0) {
-      mbar_arrive(bar(NEXT_REQ));
-    }
-    if constexpr (!HAS_O) {
-      for (int j = 0; j < n_total; j += 2, ++tile) {
-        if (stall_tile >= 0 && j >= stall_tile) { alive = false; break; }
-        if (j / 2 == max(0, n_total - NEXT_LEAD) / 2 && lane == 0) mbar_arrive(bar(NEXT_REQ));
-        const int ks = tile % KSTAGES, tiles = min(2, n_total - j);
-        int page[2] = {0, 0};
-        if (paged) {
-          page[0] = chk(p.kv_indices[page_base + j], 0, static_cast<int>(p.kv_extent), p.status);
-          if (tiles == 2) page[1] = chk(p.kv_indices[page_base + j + 1], 0, static_cast<int>(p.kv_extent), p.status);
-        }
-        alive = __all_sync(0xffffffffu, mbar_wait(bar(K_EMPTY + ks), ((tile / KSTAGES) & 1) ^ 1, abort_flag, spin_limit));
+      const int n_total = max(w.n_tiles[0], w.n_tiles[1]), head = w.head, kvh = w.kvh, kv_len = w.kv_len;
+      const int page_base = w.kv0, kv_base = w.kv0;
+      if (n_total > 0) {                                  // an item without visible keys loads nothing
+        alive = __all_sync(0xffffffffu, mbar_wait(bar(Q_EMPTY), (q_loads & 1) ^ 1, abort_flag, spin_limit));
         if (!alive) break;
+        ++q_loads;
         if (elect_one()) {
-          mbar_arrive_expect_tx(bar(K_FULL + ks), tiles * TILE_BYTES);
+          mbar_arrive_expect_tx(bar(Q_FULL), 2 * TILE_BYTES);
 #pragma unroll
-          for (int t = 0; t < 2; ++t) {
-            if (t >= tiles) break;
+          for (int x = 0; x < 2; ++x)
 #pragma unroll
-            for (int hlf = 0; hlf < NSUB; ++hlf) {       // a half of head_dim: 256 rows of 128 bytes
-              const uint32_t dst = smem_base + OFF_K + ks * PAIR_BYTES + (2 * hlf + t) * SUB_BYTES;
-              if (paged) tma_load_4d(dst, &tm_k, bar(K_FULL + ks), hlf * SUB_ELEMS, 0, kvh, page[t]);
-              else tma_load_3d(dst, &tm_k, bar(K_FULL + ks), hlf * SUB_ELEMS, kvh, kv_base + (j + t) * BN);
+            for (int hlf = 0; hlf < NSUB; ++hlf)
+              tma_load_3d(smem_base + OFF_Q + x * TILE_BYTES + hlf * SUB_BYTES, &tm_q, bar(Q_FULL), hlf * SUB_ELEMS, head,
+                          w.qo_base + w.row0 + x * BM);
+        }
+        __syncwarp();
+      } else if (lane == 0) {
+        mbar_arrive(bar(NEXT_REQ));
+      }
+      if constexpr (!HAS_O) {
+        for (int j = 0; j < n_total; j += 2, ++tile) {
+          if (stall_tile >= 0 && j >= stall_tile) { alive = false; break; }
+          if (j / 2 == max(0, n_total - NEXT_LEAD) / 2 && lane == 0) mbar_arrive(bar(NEXT_REQ));
+          const int ks = tile % KSTAGES, tiles = min(2, n_total - j);
+          int page[2] = {0, 0};
+          if (paged) {
+            page[0] = chk(p.kv_indices[page_base + j], 0, static_cast<int>(p.kv_extent), p.status);
+            if (tiles == 2) page[1] = chk(p.kv_indices[page_base + j + 1], 0, static_cast<int>(p.kv_extent), p.status);
+          }
+          alive = __all_sync(0xffffffffu, mbar_wait(bar(K_EMPTY + ks), ((tile / KSTAGES) & 1) ^ 1, abort_flag, spin_limit));
+          if (!alive) break;
+          if (elect_one()) {
+            mbar_arrive_expect_tx(bar(K_FULL + ks), tiles * TILE_BYTES);
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+              if (t >= tiles) break;
+#pragma unroll
+              for (int hlf = 0; hlf < NSUB; ++hlf) {       // a half of head_dim: 256 rows of 128 bytes
+                const uint32_t dst = smem_base + OFF_K + ks * PAIR_BYTES + (2 * hlf + t) * SUB_BYTES;
+                if (paged) tma_load_4d(dst, &tm_k, bar(K_FULL + ks), hlf * SUB_ELEMS, 0, kvh, page[t]);
+                else tma_load_3d(dst, &tm_k, bar(K_FULL + ks), hlf * SUB_ELEMS, kvh, kv_base + (j + t) * BN);
+              }
+            }
+          }
+          __syncwarp();
+        }
+      } else {
+        for (int j = 0; j < n_total && alive; ++j, ++tile) {
+          if (j == stall_tile) { alive = false; break; }    // test hook: whoever waits for this tile runs out of polls
+          if (j == max(0, n_total - NEXT_LEAD) && lane == 0) mbar_arrive(bar(NEXT_REQ));
+          const int ks = tile % KSTAGES, vs = tile % VSTAGES;
+          const int page = paged ? chk(p.kv_indices[page_base + j], 0, static_cast<int>(p.kv_extent), p.status) : 0;
+          const int valid_rows = min(BN, kv_len - j * BN);
+          const bool fix = valid_rows < BN;                 // tail tile: rows past kv_len must read as 0 in V
+          if (lane == 0) trace(3, j, 0);
+          alive = mbar_wait(bar(K_EMPTY + ks), ((tile / KSTAGES) & 1) ^ 1, abort_flag, spin_limit);
+          if (lane == 0) trace(3, j, 1);
+          if (!alive) break;
+          if (elect_one()) {
+            mbar_arrive_expect_tx(bar(K_FULL + ks), TILE_BYTES);
+#pragma unroll
+            for (int hlf = 0; hlf < NSUB; ++hlf) {
+              const uint32_t dst = smem_base + OFF_K + ks * TILE_BYTES + hlf * SUB_BYTES;
+              if (paged) tma_load_4d(dst, &tm_k, bar(K_FULL + ks), hlf * SUB_ELEMS, 0, kvh, page);
+              else tma_load_3d(dst, &tm_k, bar(K_FULL + ks), hlf * SUB_ELEMS, kvh, kv_base + j * BN);
+            }
+          }
+          __syncwarp();
+          alive = mbar_wait(bar(V_EMPTY + vs), ((tile / VSTAGES) & 1) ^ 1, abort_flag, spin_limit);
+          if (lane == 0) trace(3, j, 2);
+          if (!alive) break;
+          if (elect_one()) {
+            const uint32_t vbar = fix ? bar(V_FIX) : bar(V_FULL + vs);
+            mbar_arrive_expect_tx(vbar, TILE_BYTES);
+#pragma unroll
+            for (int hlf = 0; hlf < NSUB; ++hlf) {
+              const uint32_t dst = smem_base + OFF_V + vs * TILE_BYTES + hlf * SUB_BYTES;
+              if (paged) tma_load_4d(dst, &tm_v, vbar, hlf * SUB_ELEMS, 0, kvh, page);
+              else tma_load_3d(dst, &tm_v, vbar, hlf * SUB_ELEMS, kvh, kv_base + j * BN);
+            }
+          }
+          __syncwarp();
+          if (fix && alive) {
+            alive = mbar_wait(bar(V_FIX), fix_phase, abort_flag, spin_limit);
+            alive = __all_sync(0xffffffffu, alive);
+            fix_phase ^= 1;
+            if (alive) {
+              // whole 128-byte rows are zeroed, so the swizzle does not matter
+              unsigned char* vt = smem_gen + OFF_V + vs * TILE_BYTES;
+              for (int c = lane; c < (BN - valid_rows) * (NSUB * 8); c += 32) {
+                const int r = valid_rows + c / (NSUB * 8), ch = c % (NSUB * 8);
+                *reinterpret_cast<uint4*>(vt + (ch >> 3) * SUB_BYTES + r * 128 + (ch & 7) * 16) = make_uint4(0, 0, 0, 0);
+              }
+              fence_proxy_async_smem();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(bar(V_FULL + vs));
             }
           }
         }
-        __syncwarp();
       }
-    } else
-      for (int j = 0; j < n_total && alive; ++j, ++tile) {
-      if (j == stall_tile) { alive = false; break; }    // test hook: whoever waits for this tile runs out of polls
-      if (j == max(0, n_total - NEXT_LEAD) && lane == 0) mbar_arrive(bar(NEXT_REQ));
-      const int ks = tile % KSTAGES, vs = tile % VSTAGES;
-      const int page = paged ? chk(p.kv_indices[page_base + j], 0, static_cast<int>(p.kv_extent), p.status) : 0;
-      const int valid_rows = min(BN, kv_len - j * BN);
-      const bool fix = valid_rows < BN;                 // tail tile: rows past kv_len must read as 0 in V
-      if (lane == 0) trace(3, j, 0);
-      alive = mbar_wait(bar(K_EMPTY + ks), ((tile / KSTAGES) & 1) ^ 1, abort_flag, spin_limit);
-      if (lane == 0) trace(3, j, 1);
-      if (!alive) break;
-      if (elect_one()) {
-        mbar_arrive_expect_tx(bar(K_FULL + ks), TILE_BYTES);
-#pragma unroll
-        for (int hlf = 0; hlf < NSUB; ++hlf) {
-          const uint32_t dst = smem_base + OFF_K + ks * TILE_BYTES + hlf * SUB_BYTES;
-          if (paged) tma_load_4d(dst, &tm_k, bar(K_FULL + ks), hlf * SUB_ELEMS, 0, kvh, page);
-          else tma_load_3d(dst, &tm_k, bar(K_FULL + ks), hlf * SUB_ELEMS, kvh, kv_base + j * BN);
-        }
-      }
-      __syncwarp();
-      alive = mbar_wait(bar(V_EMPTY + vs), ((tile / VSTAGES) & 1) ^ 1, abort_flag, spin_limit);
-      if (lane == 0) trace(3, j, 2);
-      if (!alive) break;
-      if (elect_one()) {
-        const uint32_t vbar = fix ? bar(V_FIX) : bar(V_FULL + vs);
-        mbar_arrive_expect_tx(vbar, TILE_BYTES);
-#pragma unroll
-        for (int hlf = 0; hlf < NSUB; ++hlf) {
-          const uint32_t dst = smem_base + OFF_V + vs * TILE_BYTES + hlf * SUB_BYTES;
-          if (paged) tma_load_4d(dst, &tm_v, vbar, hlf * SUB_ELEMS, 0, kvh, page);
-          else tma_load_3d(dst, &tm_v, vbar, hlf * SUB_ELEMS, kvh, kv_base + j * BN);
-        }
-      }
-      __syncwarp();
-      if (fix && alive) {
-        alive = mbar_wait(bar(V_FIX), fix_phase, abort_flag, spin_limit);
-        alive = __all_sync(0xffffffffu, alive);
-        fix_phase ^= 1;
-        if (alive) {
-          // whole 128-byte rows are zeroed, so the swizzle does not matter
-          unsigned char* vt = smem_gen + OFF_V + vs * TILE_BYTES;
-          for (int c = lane; c < (BN - valid_rows) * (NSUB * 8); c += 32) {
-            const int r = valid_rows + c / (NSUB * 8), ch = c % (NSUB * 8);
-            *reinterpret_cast<uint4*>(vt + (ch >> 3) * SUB_BYTES + r * 128 + (ch & 7) * 16) = make_uint4(0, 0, 0, 0);
-          }
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar(V_FULL + vs));
-        }
-      }
-    }
     }
   } else if (warp == SCHED_WARP) {
     // =========================== scheduler: the next work item of this CTA ===========================
@@ -496,216 +497,216 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
     uint32_t s_par = 0, o_par = 0;
     Item w;
     for (uint32_t it = 0; take_item(it, w, alive); ++it) {
-    const int head = w.head, kvh = w.kvh, kv_len = w.kv_len, off = w.off;
-    const int m0 = w.row0 + x * BM;
-    const int i = m0 + r;                                // token index within the sequence
-    const bool row_ok = i < w.ql;
-    const int gtok = w.qo_base + i;
-    const int lim = row_ok ? min(i + off, kv_len - 1) : -1;
-    const int nx = x == 0 ? w.n_tiles[0] : w.n_tiles[1];
-    const float scale_log2 = p.sm_scale * kLog2e * (p.k_scale_head ? p.k_scale_head[kvh] : 1.f);
-    float m_used = -INFINITY, l_sum = 0.f;
-    float l_exact = 0.f;                                 // e4m3 only: sum of the unrounded probabilities, for the LSE
+      const int head = w.head, kvh = w.kvh, kv_len = w.kv_len, off = w.off;
+      const int m0 = w.row0 + x * BM;
+      const int i = m0 + r;                                // token index within the sequence
+      const bool row_ok = i < w.ql;
+      const int gtok = w.qo_base + i;
+      const int lim = row_ok ? min(i + off, kv_len - 1) : -1;
+      const int nx = x == 0 ? w.n_tiles[0] : w.n_tiles[1];
+      const float scale_log2 = p.sm_scale * kLog2e * (p.k_scale_head ? p.k_scale_head[kvh] : 1.f);
+      float m_used = -INFINITY, l_sum = 0.f;
+      float l_exact = 0.f;                                 // e4m3 only: sum of the unrounded probabilities, for the LSE
 
-    for (int j = 0; j < nx && alive; ++j) {
-      if (r == 0) trace(x, j, 0);
-      if (HAS_O || (j & 1) == 0) {                       // score-only: S of two tiles at a time
-        alive = __all_sync(0xffffffffu, mbar_wait(bar(S_FULL + x), s_par, abort_flag, spin_limit));
-        if (!alive) break;                               // the warp votes below: all of it goes on, or none
-        s_par ^= 1;
-      }
-      const uint32_t tS = tmem + (HAS_O ? x * BN : x * 2 * BN + (j & 1) * BN) + lane_addr;
-      tc_fence_after();
-      if (r == 0) trace(x, j, 1);
-      const int pos0 = j * BN;
-      const bool need_mask = (pos0 + BN - 1 > m0 + off) || (pos0 + BN > kv_len);
-      // ---- one read of the whole S row (128 fp32) ----
-      uint32_t sv[4][32];
-      tmem_ld32(tS, sv[0]);
-      tmem_ld32(tS + 32, sv[1]);
-      tmem_ld32(tS + 64, sv[2]);
-      tmem_ld32(tS + 96, sv[3]);
-      tmem_wait_ld();
-      if (r == 0) trace(x, j, 2);
-      if (!HAS_O && ((j & 1) || j + 1 == nx)) {          // both tiles' S are out: it may be filled again
-        tc_fence_before();
-        mbar_arrive(bar(P_FULL + x));
-      }
-      if (need_mask) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-          for (int e = 0; e < 32; ++e)
-            if (pos0 + c * 32 + e > lim) sv[c][e] = 0xff800000u;     // -inf
-      }
-      auto store_score = [&](const float mx) {
-        if (want_score && row_ok && j < p.max_k_tiles) {
-          const int64_t o = (static_cast<int64_t>(head) * p.max_k_tiles + j) * p.total_q + gtok;
-          if (p.max_score_dtype == MSA_DT_BF16) static_cast<__nv_bfloat16*>(p.max_score)[o] = __float2bfloat16_rn(mx);
-          else static_cast<float*>(p.max_score)[o] = mx;
+      for (int j = 0; j < nx && alive; ++j) {
+        if (r == 0) trace(x, j, 0);
+        if (HAS_O || (j & 1) == 0) {                       // score-only: S of two tiles at a time
+          alive = __all_sync(0xffffffffu, mbar_wait(bar(S_FULL + x), s_par, abort_flag, spin_limit));
+          if (!alive) break;                               // the warp votes below: all of it goes on, or none
+          s_par ^= 1;
         }
-      };
-      if (!has_o) {                    // score-only pass: the row max of the tile
-        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};        // four independent chains
+        const uint32_t tS = tmem + (HAS_O ? x * BN : x * 2 * BN + (j & 1) * BN) + lane_addr;
+        tc_fence_after();
+        if (r == 0) trace(x, j, 1);
+        const int pos0 = j * BN;
+        const bool need_mask = (pos0 + BN - 1 > m0 + off) || (pos0 + BN > kv_len);
+        // ---- one read of the whole S row (128 fp32) ----
+        uint32_t sv[4][32];
+        tmem_ld32(tS, sv[0]);
+        tmem_ld32(tS + 32, sv[1]);
+        tmem_ld32(tS + 64, sv[2]);
+        tmem_ld32(tS + 96, sv[3]);
+        tmem_wait_ld();
+        if (r == 0) trace(x, j, 2);
+        if (!HAS_O && ((j & 1) || j + 1 == nx)) {          // both tiles' S are out: it may be filled again
+          tc_fence_before();
+          mbar_arrive(bar(P_FULL + x));
+        }
+        if (need_mask) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+          for (int c = 0; c < 4; ++c)
 #pragma unroll
-          for (int e = 0; e < 32; e += 2)
-            m4[(e >> 1) & 3] = max3(m4[(e >> 1) & 3], __uint_as_float(sv[c][e]), __uint_as_float(sv[c][e + 1]));
-        store_score(fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])));
-        continue;
-      }
-      // P = exp2(S * scale - m) as bf16 / e4m3, written over the front of S; the row max of the tile (the
-      // max_score output, and what decides a rescale) is computed in the same pass.
-      // The special-function unit does 16 exp2 per clock per SM, a quarter of what the tensor pipe needs
-      // here, so kEmuMask selects pairs whose exp2 runs on the FMA pipe instead: round-to-nearest split
-      // x = n + f, degree-3 polynomial for 2^f (rel. error 7.5e-5, far below the rounding of P), n added
-      // into the exponent field.  All fp32 arithmetic is done on packed pairs (fma.rn.f32x2 / add.rn.f32x2).
-      float mxs[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};     // four independent chains
-      auto row_max = [&]() {
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-          for (int e = 0; e < 32; e += 2)
-            mxs[(e >> 1) & 3] = max3(mxs[(e >> 1) & 3], __uint_as_float(sv[c][e]), __uint_as_float(sv[c][e + 1]));
-      };
-      float l_rnd = 0.f, l_raw = 0.f;            // row sum of this tile: of P as stored / before rounding (e4m3)
-      auto emit_p = [&](auto with_max, const float m_ref) {
-        const uint64_t scale2 = f2_pack(scale_log2, scale_log2);
-        const uint64_t negm2 = f2_pack(-m_ref, -m_ref);
-        uint64_t lsum2 = f2_pack(0.f, 0.f), lex2 = f2_pack(0.f, 0.f);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t pk[F8 ? 8 : 16];
-          [[maybe_unused]] uint16_t held = 0;
-#pragma unroll
-          for (int e = 0; e < 32; e += 2) {
-            if constexpr (decltype(with_max)::value)
-              mxs[(e >> 1) & 3] = max3(mxs[(e >> 1) & 3], __uint_as_float(sv[c][e]), __uint_as_float(sv[c][e + 1]));
-            const uint64_t x2 = f2_fma(f2_pack(__uint_as_float(sv[c][e]), __uint_as_float(sv[c][e + 1])), scale2, negm2);
-            float p0, p1;
-            if ((kEmuMask >> ((e >> 1) & 15)) & 1) {
-              float x0, x1;
-              f2_unpack(x2, x0, x1);
-              const uint64_t xc = f2_pack(fmaxf(x0, -126.f), fmaxf(x1, -126.f));     // also maps -inf
-              const uint64_t t2 = f2_add(xc, f2_pack(12582912.f, 12582912.f));          // 1.5 * 2^23: n in the low bits
-              const uint64_t n2 = f2_add(t2, f2_pack(-12582912.f, -12582912.f));
-              const uint64_t fr = f2_fma(n2, f2_pack(-1.f, -1.f), xc);                   // f in [-0.5, 0.5]
-              uint64_t pl = f2_fma(fr, f2_pack(0.055171650f, 0.055171650f), f2_pack(0.24261113f, 0.24261113f));
-              pl = f2_fma(pl, fr, f2_pack(0.69326097f, 0.69326097f));
-              pl = f2_fma(pl, fr, f2_pack(0.99992806f, 0.99992806f));
-              float q0, q1, t0, t1;
-              f2_unpack(pl, q0, q1);
-              f2_unpack(t2, t0, t1);
-              p0 = __uint_as_float(__float_as_uint(q0) + (__float_as_uint(t0) << 23));
-              p1 = __uint_as_float(__float_as_uint(q1) + (__float_as_uint(t1) << 23));
-            } else {
-              float x0, x1;
-              f2_unpack(x2, x0, x1);
-              p0 = exp2_fast(x0);
-              p1 = exp2_fast(x1);
-            }
-            if constexpr (F8) {
-              // O is normalised by the sum of the probabilities as the MMA sees them (see the decode kernel);
-              // the LSE reports the sum before rounding
-              lex2 = f2_add(lex2, f2_pack(p0, p1));
-              const uint16_t pr = __nv_cvt_float2_to_fp8x2(make_float2(p0, p1), __NV_SATFINITE, __NV_E4M3);
-              const float2 rr = e4m3x2_to_float2(pr);
-              lsum2 = f2_add(lsum2, f2_pack(rr.x, rr.y));
-              if (e & 2) pk[e >> 2] = static_cast<uint32_t>(held) | (static_cast<uint32_t>(pr) << 16);
-              else held = pr;
-            } else {
-              lsum2 = f2_add(lsum2, f2_pack(p0, p1));
-              pk[e >> 1] = pack2<false>(p0, p1);
-            }
+            for (int e = 0; e < 32; ++e)
+              if (pos0 + c * 32 + e > lim) sv[c][e] = 0xff800000u;     // -inf
+        }
+        auto store_score = [&](const float mx) {
+          if (want_score && row_ok && j < p.max_k_tiles) {
+            const int64_t o = (static_cast<int64_t>(head) * p.max_k_tiles + j) * p.total_q + gtok;
+            if (p.max_score_dtype == MSA_DT_BF16) static_cast<__nv_bfloat16*>(p.max_score)[o] = __float2bfloat16_rn(mx);
+            else static_cast<float*>(p.max_score)[o] = mx;
           }
-          if constexpr (F8) tmem_st8(tS + c * 8, pk);
-          else tmem_st16(tS + c * 16, pk);
+        };
+        if (!has_o) {                    // score-only pass: the row max of the tile
+          float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};        // four independent chains
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int e = 0; e < 32; e += 2)
+              m4[(e >> 1) & 3] = max3(m4[(e >> 1) & 3], __uint_as_float(sv[c][e]), __uint_as_float(sv[c][e + 1]));
+          store_score(fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])));
+          continue;
         }
-        float l0, l1;
-        f2_unpack(lsum2, l0, l1);
-        l_rnd = l0 + l1;
-        if constexpr (F8) { f2_unpack(lex2, l0, l1); l_raw = l0 + l1; }
-      };
-      // Every tile but the first writes P with the running max while it finds its own max: the max does
-      // not sit between the S read and the exponentials, and the guess holds unless the row's max grows
-      // by more than the rescale threshold (then P is written again below).
-      // (bf16 only: with e4m3 operands the kernel measured 6 % slower this way.)
-      const bool guess = !F8 && j > 0;                              // warp-uniform
-      const float m_guess = ((m_used == -INFINITY) ? 0.f : m_used) - kPOffset;
-      if (guess) emit_p(std::true_type{}, m_guess);
-      else row_max();
-      const float mx = fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3]));
-      store_score(mx);
-      // ---- running max with lazy rescale ----
-      const float m_cand = fmaxf(m_used, mx * scale_log2);
-      // false for (-inf) - (-inf) = NaN; true for a row whose first visible key is in this tile (its guess
-      // was made without a max)
-      const bool bump = (m_cand - m_used) > kRescaleThreshold;
-      if (!guess || __any_sync(0xffffffffu, bump)) {
-        float factor = 1.f;
-        if (bump) { factor = exp2_fast(m_used - m_cand); m_used = m_cand; l_sum *= factor; l_exact *= factor; }
-        if (j > 0 && __any_sync(0xffffffffu, bump)) {
+        // P = exp2(S * scale - m) as bf16 / e4m3, written over the front of S; the row max of the tile (the
+        // max_score output, and what decides a rescale) is computed in the same pass.
+        // The special-function unit does 16 exp2 per clock per SM, a quarter of what the tensor pipe needs
+        // here, so kEmuMask selects pairs whose exp2 runs on the FMA pipe instead: round-to-nearest split
+        // x = n + f, degree-3 polynomial for 2^f (rel. error 7.5e-5, far below the rounding of P), n added
+        // into the exponent field.  All fp32 arithmetic is done on packed pairs (fma.rn.f32x2 / add.rn.f32x2).
+        float mxs[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};     // four independent chains
+        auto row_max = [&]() {
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int e = 0; e < 32; e += 2)
+              mxs[(e >> 1) & 3] = max3(mxs[(e >> 1) & 3], __uint_as_float(sv[c][e]), __uint_as_float(sv[c][e + 1]));
+        };
+        float l_rnd = 0.f, l_raw = 0.f;            // row sum of this tile: of P as stored / before rounding (e4m3)
+        auto emit_p = [&](auto with_max, const float m_ref) {
+          const uint64_t scale2 = f2_pack(scale_log2, scale_log2);
+          const uint64_t negm2 = f2_pack(-m_ref, -m_ref);
+          uint64_t lsum2 = f2_pack(0.f, 0.f), lex2 = f2_pack(0.f, 0.f);
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            uint32_t v[32];
+            uint32_t pk[F8 ? 8 : 16];
+            [[maybe_unused]] uint16_t held = 0;
+#pragma unroll
+            for (int e = 0; e < 32; e += 2) {
+              if constexpr (decltype(with_max)::value)
+                mxs[(e >> 1) & 3] = max3(mxs[(e >> 1) & 3], __uint_as_float(sv[c][e]), __uint_as_float(sv[c][e + 1]));
+              const uint64_t x2 = f2_fma(f2_pack(__uint_as_float(sv[c][e]), __uint_as_float(sv[c][e + 1])), scale2, negm2);
+              float p0, p1;
+              if ((kEmuMask >> ((e >> 1) & 15)) & 1) {
+                float x0, x1;
+                f2_unpack(x2, x0, x1);
+                const uint64_t xc = f2_pack(fmaxf(x0, -126.f), fmaxf(x1, -126.f));     // also maps -inf
+                const uint64_t t2 = f2_add(xc, f2_pack(12582912.f, 12582912.f));          // 1.5 * 2^23: n in the low bits
+                const uint64_t n2 = f2_add(t2, f2_pack(-12582912.f, -12582912.f));
+                const uint64_t fr = f2_fma(n2, f2_pack(-1.f, -1.f), xc);                   // f in [-0.5, 0.5]
+                uint64_t pl = f2_fma(fr, f2_pack(0.055171650f, 0.055171650f), f2_pack(0.24261113f, 0.24261113f));
+                pl = f2_fma(pl, fr, f2_pack(0.69326097f, 0.69326097f));
+                pl = f2_fma(pl, fr, f2_pack(0.99992806f, 0.99992806f));
+                float q0, q1, t0, t1;
+                f2_unpack(pl, q0, q1);
+                f2_unpack(t2, t0, t1);
+                p0 = __uint_as_float(__float_as_uint(q0) + (__float_as_uint(t0) << 23));
+                p1 = __uint_as_float(__float_as_uint(q1) + (__float_as_uint(t1) << 23));
+              } else {
+                float x0, x1;
+                f2_unpack(x2, x0, x1);
+                p0 = exp2_fast(x0);
+                p1 = exp2_fast(x1);
+              }
+              if constexpr (F8) {
+                // O is normalised by the sum of the probabilities as the MMA sees them (see the decode kernel);
+                // the LSE reports the sum before rounding
+                lex2 = f2_add(lex2, f2_pack(p0, p1));
+                const uint16_t pr = __nv_cvt_float2_to_fp8x2(make_float2(p0, p1), __NV_SATFINITE, __NV_E4M3);
+                const float2 rr = e4m3x2_to_float2(pr);
+                lsum2 = f2_add(lsum2, f2_pack(rr.x, rr.y));
+                if (e & 2) pk[e >> 2] = static_cast<uint32_t>(held) | (static_cast<uint32_t>(pr) << 16);
+                else held = pr;
+              } else {
+                lsum2 = f2_add(lsum2, f2_pack(p0, p1));
+                pk[e >> 1] = pack2<false>(p0, p1);
+              }
+            }
+            if constexpr (F8) tmem_st8(tS + c * 8, pk);
+            else tmem_st16(tS + c * 16, pk);
+          }
+          float l0, l1;
+          f2_unpack(lsum2, l0, l1);
+          l_rnd = l0 + l1;
+          if constexpr (F8) { f2_unpack(lex2, l0, l1); l_raw = l0 + l1; }
+        };
+        // Every tile but the first writes P with the running max while it finds its own max: the max does
+        // not sit between the S read and the exponentials, and the guess holds unless the row's max grows
+        // by more than the rescale threshold (then P is written again below).
+        // (bf16 only: with e4m3 operands the kernel measured 6 % slower this way.)
+        const bool guess = !F8 && j > 0;                              // warp-uniform
+        const float m_guess = ((m_used == -INFINITY) ? 0.f : m_used) - kPOffset;
+        if (guess) emit_p(std::true_type{}, m_guess);
+        else row_max();
+        const float mx = fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3]));
+        store_score(mx);
+        // ---- running max with lazy rescale ----
+        const float m_cand = fmaxf(m_used, mx * scale_log2);
+        // false for (-inf) - (-inf) = NaN; true for a row whose first visible key is in this tile (its guess
+        // was made without a max)
+        const bool bump = (m_cand - m_used) > kRescaleThreshold;
+        if (!guess || __any_sync(0xffffffffu, bump)) {
+          float factor = 1.f;
+          if (bump) { factor = exp2_fast(m_used - m_cand); m_used = m_cand; l_sum *= factor; l_exact *= factor; }
+          if (j > 0 && __any_sync(0xffffffffu, bump)) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              uint32_t v[32];
+              tmem_ld32(tO + c * 32, v);
+              tmem_wait_ld();
+#pragma unroll
+              for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) * factor);
+              tmem_st32(tO + c * 32, v);
+            }
+          }
+          if (r == 0) trace(x, j, 3);
+          emit_p(std::false_type{}, ((m_used == -INFINITY) ? 0.f : m_used) - kPOffset);
+        }
+        l_sum += l_rnd;
+        if constexpr (F8) l_exact += l_raw;
+        if (r == 0) trace(x, j, 4);
+        tmem_wait_st();
+        tc_fence_before();
+        mbar_arrive(bar(P_FULL + x));
+        if (r == 0) trace(x, j, 5);
+      }
+
+      // ---- epilogue ----
+      if (alive && nx > 0 && has_o) {
+        alive = __all_sync(0xffffffffu, mbar_wait(bar(O_FULL + x), o_par, abort_flag, spin_limit));
+        o_par ^= 1;
+      }
+      if (alive && has_o) {
+        tc_fence_after();
+        const float vsh = p.v_scale_head ? p.v_scale_head[kvh] : 1.f;
+        const float inv = l_sum > 0.f ? p.out_scale * vsh / l_sum : 0.f;
+        __nv_bfloat16* dst = p.out ? static_cast<__nv_bfloat16*>(p.out) + static_cast<int64_t>(gtok) * p.out_stride_tok +
+                                         static_cast<int64_t>(head) * p.out_stride_head
+                                   : nullptr;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t v[32];
+          if (nx > 0) {
             tmem_ld32(tO + c * 32, v);
             tmem_wait_ld();
+          } else {
 #pragma unroll
-            for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) * factor);
-            tmem_st32(tO + c * 32, v);
+            for (int e = 0; e < 32; ++e) v[e] = 0u;
+          }
+          if (row_ok && dst) {
+#pragma unroll
+            for (int e = 0; e < 32; e += 8) {
+              uint4 o4;
+              o4.x = pack2<false>(__uint_as_float(v[e]) * inv, __uint_as_float(v[e + 1]) * inv);
+              o4.y = pack2<false>(__uint_as_float(v[e + 2]) * inv, __uint_as_float(v[e + 3]) * inv);
+              o4.z = pack2<false>(__uint_as_float(v[e + 4]) * inv, __uint_as_float(v[e + 5]) * inv);
+              o4.w = pack2<false>(__uint_as_float(v[e + 6]) * inv, __uint_as_float(v[e + 7]) * inv);
+              *reinterpret_cast<uint4*>(dst + c * 32 + e) = o4;
+            }
           }
         }
-        if (r == 0) trace(x, j, 3);
-        emit_p(std::false_type{}, ((m_used == -INFINITY) ? 0.f : m_used) - kPOffset);
+        if (row_ok && p.lse)
+          p.lse[static_cast<int64_t>(gtok) * p.num_qo_heads + head] =
+              l_sum > 0.f ? (m_used - kPOffset) * kLn2 + __logf(F8 ? l_exact : l_sum) : -INFINITY;
       }
-      l_sum += l_rnd;
-      if constexpr (F8) l_exact += l_raw;
-      if (r == 0) trace(x, j, 4);
-      tmem_wait_st();
-      tc_fence_before();
-      mbar_arrive(bar(P_FULL + x));
-      if (r == 0) trace(x, j, 5);
-    }
-
-    // ---- epilogue ----
-    if (alive && nx > 0 && has_o) {
-      alive = __all_sync(0xffffffffu, mbar_wait(bar(O_FULL + x), o_par, abort_flag, spin_limit));
-      o_par ^= 1;
-    }
-    if (alive && has_o) {
-      tc_fence_after();
-      const float vsh = p.v_scale_head ? p.v_scale_head[kvh] : 1.f;
-      const float inv = l_sum > 0.f ? p.out_scale * vsh / l_sum : 0.f;
-      __nv_bfloat16* dst = p.out ? static_cast<__nv_bfloat16*>(p.out) + static_cast<int64_t>(gtok) * p.out_stride_tok +
-                                       static_cast<int64_t>(head) * p.out_stride_head
-                                 : nullptr;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t v[32];
-        if (nx > 0) {
-          tmem_ld32(tO + c * 32, v);
-          tmem_wait_ld();
-        } else {
-#pragma unroll
-          for (int e = 0; e < 32; ++e) v[e] = 0u;
-        }
-        if (row_ok && dst) {
-#pragma unroll
-          for (int e = 0; e < 32; e += 8) {
-            uint4 o4;
-            o4.x = pack2<false>(__uint_as_float(v[e]) * inv, __uint_as_float(v[e + 1]) * inv);
-            o4.y = pack2<false>(__uint_as_float(v[e + 2]) * inv, __uint_as_float(v[e + 3]) * inv);
-            o4.z = pack2<false>(__uint_as_float(v[e + 4]) * inv, __uint_as_float(v[e + 5]) * inv);
-            o4.w = pack2<false>(__uint_as_float(v[e + 6]) * inv, __uint_as_float(v[e + 7]) * inv);
-            *reinterpret_cast<uint4*>(dst + c * 32 + e) = o4;
-          }
-        }
-      }
-      if (row_ok && p.lse)
-        p.lse[static_cast<int64_t>(gtok) * p.num_qo_heads + head] =
-            l_sum > 0.f ? (m_used - kPOffset) * kLn2 + __logf(F8 ? l_exact : l_sum) : -INFINITY;
-    }
     }
   }
 
