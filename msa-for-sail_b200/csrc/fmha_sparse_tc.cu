@@ -530,6 +530,10 @@ sparse_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
     int ent = entry_of(0);
     for (int c = 0; c < n_chunks && alive; ++c) {
       const int x = c % NQBUF, u = c / NQBUF;
+      // A warp without a row in the (last, partial) chunk must not wait for its buffer: Q K^T of that chunk does not need
+      // the warp and may give the buffer back first, and the parity the warp waits for would then never come.  The first
+      // warp always has a row, and announces the chunk's bytes.
+      if ((warp - GATHER_WARP0) / upt >= min(tpc, item.z - (item.y + c * tpc))) break;
       if (gt == 0) trace(4, c, 0);
       alive = mbar_wait(bar(Q_EMPTY + x), (u & 1) ^ 1, abort_flag);   // Q K^T of chunk c - 3 has read the buffer
       if (!alive) break;

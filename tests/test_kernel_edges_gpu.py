@@ -173,6 +173,41 @@ def test_sparse_merge_edges(kbn, hq, hk, T):
     assert (lse - ref_lse)[seen].abs().max() <= 2e-3
 
 
+@pytest.mark.parametrize("dtype,hq,hk", [(torch.float8_e4m3fn, 16, 1), (torch.bfloat16, 8, 1)])
+def test_sparse_prefill_partial_chunks(dtype, hq, hk):
+    """Page lists whose last chunk has one token, so that two of the three loader warps have no row in it: a loader that
+    waited for that chunk's buffer all the same could miss its phase and run into the limit of its wait."""
+    import msa_for_sail as msa
+    from msa_for_sail import api
+    g = gen(77)
+    pages, tpc = 64, 128 * hk // hq
+    # every page is selected by the same number of tokens: one more than a multiple of a chunk's
+    per_page = 5 * tpc + 1
+    T = pages * per_page // 4
+    kv = [pages * 128 + T]
+    order = torch.randperm(pages * per_page, generator=g)[:T * 4] % pages
+    bi = order.view(T, 4)
+    for c in range(1, 4):                                    # four different pages a token
+        while True:
+            clash = (bi[:, :c] == bi[:, c:c + 1]).any(1)
+            if not clash.any():
+                break
+            bi[clash, c] = (bi[clash, c] + 1) % pages
+    bi = bi.sort(1).values.to(torch.int32).view(T, 1, 4)
+    q = randn_bf16(g, T, hq, 128).to(dtype).to(DEV)
+    kp, vp, table = make_paged(g, kv, hk, 128, dtype=dtype)
+    kp, vp, table, bi = kp.to(DEV), vp.to(DEV), table.to(DEV), bi.to(DEV)
+    plan = msa.fmha_sail_plan(i32([T]), i32(kv), hq, num_kv_heads=hk, page_size=128, kv_block_num=4,
+                              use_fp8_kvcache=dtype != torch.bfloat16)
+    assert plan[3]["sparse_tc_preferred"]
+    first, _ = msa.fmha_sail(q, kp, vp, plan, kv_indices=table, kv_block_indexes=bi)
+    out = torch.empty_like(first)
+    for _ in range(300):
+        msa.fmha_sail(q, kp, vp, plan, kv_indices=table, kv_block_indexes=bi, out=out)
+    assert api.last_status() == 0
+    assert torch.equal(out, first)
+
+
 # ---- planning on the device ----
 @pytest.mark.parametrize("batch", [1, 31, 32, 33, 256, 257, 600])
 def test_device_plan_prefix_sums(batch):
