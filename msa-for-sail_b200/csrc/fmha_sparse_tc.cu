@@ -496,8 +496,7 @@ sparse_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
       }
       __syncwarp();
       if (fix) {
-        alive = mbar_wait(bar(V_FIX), 0, abort_flag);
-        alive = __all_sync(0xffffffffu, alive);
+        alive = mbar_wait_warp(bar(V_FIX), 0, abort_flag);
         if (alive) {
           unsigned char* vt = smem_gen + OFF_V;
           for (int c = lane; c < (BN - valid_rows) * (NSUB * 8); c += 32) {
@@ -535,7 +534,9 @@ sparse_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
       // warp always has a row, and announces the chunk's bytes.
       if ((warp - GATHER_WARP0) / upt >= min(tpc, item.z - (item.y + c * tpc))) break;
       if (gt == 0) trace(4, c, 0);
-      alive = mbar_wait(bar(Q_EMPTY + x), (u & 1) ^ 1, abort_flag);   // Q K^T of chunk c - 3 has read the buffer
+      // Q K^T of chunk c - NQBUF has read the buffer.  The same holds for a lane as for a warp: most lanes have no unit, and
+      // none may still wait here when the others' rows let Q K^T of this chunk turn the phase.
+      alive = mbar_wait_warp(bar(Q_EMPTY + x), (u & 1) ^ 1, abort_flag);
       if (!alive) break;
       const int e0 = item.y + c * tpc;
       const int ntok = min(tpc, item.z - e0);

@@ -59,6 +59,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   *abort_flag = 1;
   return false;
 }
+// The wait of a warp that goes on as one: every lane has seen the phase, or none goes on.  A lane on its own could lag
+// behind its neighbours until the phase it waits for has come and gone (two phases of a barrier look alike), or give up
+// where they went on, and leave them in a warp-wide instruction.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag,
+                                               uint32_t limit = kSpinLimit) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, limit));
+}
 
 // One lane of a converged warp (the compiler can keep the operands of the instructions issued
 // under this predicate in uniform registers).
