@@ -293,7 +293,7 @@ decode_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
       const int valid_rows = min(TK, kv_len - key0);
       const bool fix = valid_rows < TK;
       if (do_k) {
-        alive = mbar_wait(bar(K_EMPTY + st), ((j / STAGES) & 1) ^ 1, abort_flag);
+        alive = mbar_wait_warp(bar(K_EMPTY + st), ((j / STAGES) & 1) ^ 1, abort_flag);
         if (!alive) break;
         if (elect_one()) {
           mbar_arrive_expect_tx(bar(K_FULL + st), TILE_BYTES);
@@ -305,7 +305,7 @@ decode_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
         __syncwarp();
       }
       if (!do_v) continue;
-      alive = mbar_wait(bar(V_EMPTY + st), ((j / STAGES) & 1) ^ 1, abort_flag);
+      alive = mbar_wait_warp(bar(V_EMPTY + st), ((j / STAGES) & 1) ^ 1, abort_flag);
       if (!alive) break;
       if (elect_one()) {
         const uint32_t vbar = fix ? bar(V_FIX) : bar(V_FULL + st);
@@ -316,8 +316,7 @@ decode_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
       }
       __syncwarp();
       if (fix) {                                             // rows past kv_len must read as 0 in V
-        alive = mbar_wait(bar(V_FIX), fix_phase, abort_flag);
-        alive = __all_sync(0xffffffffu, alive);
+        alive = mbar_wait_warp(bar(V_FIX), fix_phase, abort_flag);
         fix_phase ^= 1;
         if (alive) {
           unsigned char* vt = smem_gen + OFF_V + st * TILE_BYTES;
@@ -363,17 +362,17 @@ decode_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
     // tile j.  One buffer (dual): issued after P_j V_j, which is what frees the buffer.
     auto next_qk = [&](int j, bool& alive) {
       const int st = (j + 1) % STAGES;
-      alive = mbar_wait(bar(K_FULL + st), ((j + 1) / STAGES) & 1, abort_flag);
+      alive = mbar_wait_warp(bar(K_FULL + st), ((j + 1) / STAGES) & 1, abort_flag);
       // score-only pass: no P.V orders the reuse of the S buffer, wait for its reader instead
       if (alive && !has_o && j + 1 >= NBUF)
-        alive = mbar_wait(bar(P_FULL + (j + 1) % NBUF), ((j + 1 - NBUF) / NBUF) & 1, abort_flag);
+        alive = mbar_wait_warp(bar(P_FULL + (j + 1) % NBUF), ((j + 1 - NBUF) / NBUF) & 1, abort_flag);
       if (!alive) return;
       tc_fence_after();
       if (elect_one()) { issue_qk(j + 1); mma_commit(bar(S_FULL + (j + 1) % NBUF)); mma_commit(bar(K_EMPTY + st)); }
       __syncwarp();
     };
-    bool alive = n_tiles > 0 ? mbar_wait(bar(Q_FULL), 0, abort_flag) : true;
-    if (alive && n_tiles > 0) alive = mbar_wait(bar(K_FULL + 0), 0, abort_flag);
+    bool alive = n_tiles > 0 ? mbar_wait_warp(bar(Q_FULL), 0, abort_flag) : true;
+    if (alive && n_tiles > 0) alive = mbar_wait_warp(bar(K_FULL + 0), 0, abort_flag);
     if (alive && n_tiles > 0) {
       tc_fence_after();
       if (elect_one()) { issue_qk(0); mma_commit(bar(S_FULL + 0)); mma_commit(bar(K_EMPTY + 0)); }
@@ -382,8 +381,8 @@ decode_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
     for (int j = 0; j < n_tiles && alive; ++j) {
       if (NBUF == 2 && j + 1 < n_tiles) { next_qk(j, alive); if (!alive) break; }
       if (has_o) {
-        alive = mbar_wait(bar(V_FULL + j % STAGES), (j / STAGES) & 1, abort_flag);
-        if (alive) alive = mbar_wait(bar(P_FULL + j % NBUF), (j / NBUF) & 1, abort_flag);
+        alive = mbar_wait_warp(bar(V_FULL + j % STAGES), (j / STAGES) & 1, abort_flag);
+        if (alive) alive = mbar_wait_warp(bar(P_FULL + j % NBUF), (j / NBUF) & 1, abort_flag);
         if (!alive) break;
         tc_fence_after();
         if (elect_one()) {
@@ -459,7 +458,7 @@ decode_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
       // quadrant `warp` owns key columns [32 warp, 32 warp + 32) of every tile
       for (int j = 0; j < n_tiles && alive; ++j) {
         const uint32_t tS = tmem + (j % NBUF) * TK + lane_addr;
-        alive = mbar_wait(bar(S_FULL + j % NBUF), (j / NBUF) & 1, abort_flag);
+        alive = mbar_wait_warp(bar(S_FULL + j % NBUF), (j / NBUF) & 1, abort_flag);
         if (!alive) break;
         if (trace && j == 12) trace[4] = clock64() - clk0;       // S of tile 12 ready
         if (trace && j == 13) trace[14] = clock64() - clk0;
@@ -486,7 +485,7 @@ decode_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
         float factor = 1.f;
         if (bump) { factor = exp2_fast(m_used - m_cand); m_used = m_cand; l_sum *= factor; }
         if (j > 0 && __any_sync(0xffffffffu, bump)) {
-          alive = mbar_wait(bar(PV_DONE), (j - 1) & 1, abort_flag);
+          alive = mbar_wait_warp(bar(PV_DONE), (j - 1) & 1, abort_flag);
           if (!alive) break;
           tc_fence_after();
 #pragma unroll
@@ -554,7 +553,7 @@ decode_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
     } else {
     for (int j = 0; j < n_tiles && alive; ++j) {
       const uint32_t tS = tmem + (j % NBUF) * TK + lane_addr;
-      alive = mbar_wait(bar(S_FULL + j % NBUF), (j / NBUF) & 1, abort_flag);
+      alive = mbar_wait_warp(bar(S_FULL + j % NBUF), (j / NBUF) & 1, abort_flag);
       if (!alive) break;
       tc_fence_after();
       const int pos0 = tile_key0(j);
@@ -597,7 +596,7 @@ decode_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
       if (bump) { factor = exp2_fast(m_used - m_cand); m_used = m_cand; l_sum *= factor; }
       if (j > 0 && __any_sync(0xffffffffu, bump)) {
         // O may still be the target of P_{j-1} V_{j-1}: wait for that MMA before touching it
-        alive = mbar_wait(bar(PV_DONE), (j - 1) & 1, abort_flag);
+        alive = mbar_wait_warp(bar(PV_DONE), (j - 1) & 1, abort_flag);
         if (!alive) break;
         tc_fence_after();
 #pragma unroll
@@ -651,7 +650,7 @@ decode_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
     }
 
     // ---- epilogue ----
-    if (alive && n_tiles > 0 && has_o) alive = mbar_wait(bar(O_DONE), 0, abort_flag);
+    if (alive && n_tiles > 0 && has_o) alive = mbar_wait_warp(bar(O_DONE), 0, abort_flag);
     if (trace) trace[9] = clock64() - clk0;
     if constexpr (QUAD) {
       // every MMA and every TMA load of this CTA has completed: the K ring is free to stage the
@@ -659,7 +658,6 @@ decode_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
       float* stage = reinterpret_cast<float*>(smem_gen + OFF_K);              // [4][nrows][STAGE_LD]
       float* st_m = reinterpret_cast<float*>(smem_gen + OFF_V);               // [4][QUAD_MAX_ROWS]
       float* st_l = st_m + 4 * QUAD_MAX_ROWS;
-      alive = __all_sync(0xffffffffu, alive);
       if (alive && has_o) {
         tc_fence_after();
 #pragma unroll

@@ -602,7 +602,7 @@ sparse_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
     // from its warpgroup and O of chunk d - 1 drained).  Each has waits of its own -- the Q gather on
     // one side, the drain of O on the other -- so the warp polls both and issues whichever is ready
     // instead of blocking on one in a fixed order.
-    bool alive = mbar_wait(bar(K_FULL), 0, abort_flag);
+    bool alive = mbar_wait_warp(bar(K_FULL), 0, abort_flag);
     int pv = 0, qk = 0;
     uint32_t idle = 0;
     bool v_ready = false;
@@ -612,11 +612,11 @@ sparse_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
         bool rdy = mbar_test(bar(P_FULL + pv % NSBUF), (pv / NSBUF) & 1);
         if (rdy && pv > 0) rdy = mbar_test(bar(O_FREE), (pv - 1) & 1);
         if (__any_sync(0xffffffffu, rdy)) {
-          if (!v_ready) { alive = mbar_wait(bar(V_FULL), 0, abort_flag); v_ready = true; if (!alive) break; }
+          if (!v_ready) { alive = mbar_wait_warp(bar(V_FULL), 0, abort_flag); v_ready = true; if (!alive) break; }
           // every lane observes the completed phases itself (returns at once): the issuing lane may
           // not be one that saw them
-          alive = mbar_wait(bar(P_FULL + pv % NSBUF), (pv / NSBUF) & 1, abort_flag);
-          if (alive && pv > 0) alive = mbar_wait(bar(O_FREE), (pv - 1) & 1, abort_flag);
+          alive = mbar_wait_warp(bar(P_FULL + pv % NSBUF), (pv / NSBUF) & 1, abort_flag);
+          if (alive && pv > 0) alive = mbar_wait_warp(bar(O_FREE), (pv - 1) & 1, abort_flag);
           if (!alive) break;
           tc_fence_after();
           if (lane == 0) trace(3, pv, 4);
@@ -633,7 +633,7 @@ sparse_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
       if (qk < n_chunks && qk < pv + NSBUF) {
         const int x = qk % NQBUF;
         if (__any_sync(0xffffffffu, mbar_test(bar(Q_FULL + x), (qk / NQBUF) & 1))) {
-          alive = mbar_wait(bar(Q_FULL + x), (qk / NQBUF) & 1, abort_flag);
+          alive = mbar_wait_warp(bar(Q_FULL + x), (qk / NQBUF) & 1, abort_flag);
           if (!alive) break;
           tc_fence_after();
           if (lane == 0) trace(3, qk, 2);
@@ -652,7 +652,7 @@ sparse_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
       } else if (++idle >= kSpinLimit) {
         *abort_flag = 1;
         alive = false;
-      } else if ((idle & 255u) == 255u && *abort_flag) {
+      } else if ((idle & 255u) == 255u && __any_sync(0xffffffffu, *abort_flag != 0)) {
         alive = false;
       }
     }
@@ -689,7 +689,7 @@ sparse_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
       const int tok = entry >> 5;
       const int lim = row_ok ? min(tok - qo_base + off, kv_len - 1) : -1;
       if (r == 0) trace(x, c, 0);
-      alive = mbar_wait(bar(S_FULL + x), u & 1, abort_flag);
+      alive = mbar_wait_warp(bar(S_FULL + x), u & 1, abort_flag);
       if (!alive) break;
       tc_fence_after();
       if (r == 0) trace(x, c, 1);
@@ -774,8 +774,8 @@ sparse_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
       // the bulk copies of chunk c - 3 have left this warp's staging rows
       if (issuer) tma_store_wait_read();
       __syncwarp();
-      alive = mbar_wait(bar(O_FULL + x), u & 1, abort_flag);
-      if (!__all_sync(0xffffffffu, alive)) { alive = false; break; }
+      alive = mbar_wait_warp(bar(O_FULL + x), u & 1, abort_flag);
+      if (!alive) break;
       tc_fence_after();
       if (r == 0) trace(x, c, 5);
       tmem_ld32(tO, sv[0]);

@@ -175,11 +175,9 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
 
   // item number `it` of this CTA, for a whole warp: false when there is none or a wait of any lane gave up
   auto take_item = [&](uint32_t it, Item& w, bool alive) -> bool {
-    if (!__all_sync(0xffffffffu, alive)) return false;
+    if (!alive) return false;
     const uint32_t slot = it & 1;
-    bool ok = mbar_wait(bar(ITEM_FULL + slot), (it >> 1) & 1, abort_flag, spin_limit);
-    ok = __all_sync(0xffffffffu, ok);
-    if (!ok) return false;
+    if (!mbar_wait_warp(bar(ITEM_FULL + slot), (it >> 1) & 1, abort_flag, spin_limit)) return false;
     w = items[slot];
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(ITEM_EMPTY + slot));
@@ -200,7 +198,7 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
       const int n_total = max(w.n_tiles[0], w.n_tiles[1]), head = w.head, kvh = w.kvh, kv_len = w.kv_len;
       const int page_base = w.kv0, kv_base = w.kv0;
       if (n_total > 0) {                                  // an item without visible keys loads nothing
-        alive = __all_sync(0xffffffffu, mbar_wait(bar(Q_EMPTY), (q_loads & 1) ^ 1, abort_flag, spin_limit));
+        alive = mbar_wait_warp(bar(Q_EMPTY), (q_loads & 1) ^ 1, abort_flag, spin_limit);
         if (!alive) break;
         ++q_loads;
         if (elect_one()) {
@@ -226,7 +224,7 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
             page[0] = chk(p.kv_indices[page_base + j], 0, static_cast<int>(p.kv_extent), p.status);
             if (tiles == 2) page[1] = chk(p.kv_indices[page_base + j + 1], 0, static_cast<int>(p.kv_extent), p.status);
           }
-          alive = __all_sync(0xffffffffu, mbar_wait(bar(K_EMPTY + ks), ((tile / KSTAGES) & 1) ^ 1, abort_flag, spin_limit));
+          alive = mbar_wait_warp(bar(K_EMPTY + ks), ((tile / KSTAGES) & 1) ^ 1, abort_flag, spin_limit);
           if (!alive) break;
           if (elect_one()) {
             mbar_arrive_expect_tx(bar(K_FULL + ks), tiles * TILE_BYTES);
@@ -252,7 +250,7 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
           const int valid_rows = min(BN, kv_len - j * BN);
           const bool fix = valid_rows < BN;                 // tail tile: rows past kv_len must read as 0 in V
           if (lane == 0) trace(3, j, 0);
-          alive = mbar_wait(bar(K_EMPTY + ks), ((tile / KSTAGES) & 1) ^ 1, abort_flag, spin_limit);
+          alive = mbar_wait_warp(bar(K_EMPTY + ks), ((tile / KSTAGES) & 1) ^ 1, abort_flag, spin_limit);
           if (lane == 0) trace(3, j, 1);
           if (!alive) break;
           if (elect_one()) {
@@ -265,7 +263,7 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
             }
           }
           __syncwarp();
-          alive = mbar_wait(bar(V_EMPTY + vs), ((tile / VSTAGES) & 1) ^ 1, abort_flag, spin_limit);
+          alive = mbar_wait_warp(bar(V_EMPTY + vs), ((tile / VSTAGES) & 1) ^ 1, abort_flag, spin_limit);
           if (lane == 0) trace(3, j, 2);
           if (!alive) break;
           if (elect_one()) {
@@ -280,8 +278,7 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
           }
           __syncwarp();
           if (fix && alive) {
-            alive = mbar_wait(bar(V_FIX), fix_phase, abort_flag, spin_limit);
-            alive = __all_sync(0xffffffffu, alive);
+            alive = mbar_wait_warp(bar(V_FIX), fix_phase, abort_flag, spin_limit);
             fix_phase ^= 1;
             if (alive) {
               // whole 128-byte rows are zeroed, so the swizzle does not matter
@@ -308,8 +305,7 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
     int idx = static_cast<int>(blockIdx.x);
     bool alive = true;
     for (uint32_t it = 0; alive; ++it) {
-      if (it >= 2) alive = mbar_wait(bar(ITEM_EMPTY + (it & 1)), ((it >> 1) - 1) & 1, abort_flag, spin_limit);
-      alive = __all_sync(0xffffffffu, alive);
+      if (it >= 2) alive = mbar_wait_warp(bar(ITEM_EMPTY + (it & 1)), ((it >> 1) - 1) & 1, abort_flag, spin_limit);
       if (!alive) break;
       Item w;
       w.valid = idx >= 0;
@@ -341,7 +337,7 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
       }
       __syncwarp();
       if (idx < 0) break;
-      alive = __all_sync(0xffffffffu, mbar_wait(bar(NEXT_REQ), it & 1, abort_flag, spin_limit));
+      alive = mbar_wait_warp(bar(NEXT_REQ), it & 1, abort_flag, spin_limit);
       if (!alive) break;
       if (lane == 0) {
         mbar_arrive_expect_tx(bar(NEXT_FULL), 16);
@@ -397,18 +393,17 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
     for (uint32_t it = 0; take_item(it, w, alive); ++it) {
       const int n_total = max(w.n_tiles[0], w.n_tiles[1]);
       if (n_total == 0) continue;
-      alive = mbar_wait(bar(Q_FULL), q_loads & 1, abort_flag, spin_limit);
+      alive = mbar_wait_warp(bar(Q_FULL), q_loads & 1, abort_flag, spin_limit);
       ++q_loads;
       if constexpr (!HAS_O) {
         constexpr uint32_t IDESC_PAIR = F8 ? idesc_e4m3(BM, 2 * BN, false, false) : idesc_bf16(BM, 2 * BN, false, false);
         for (int j = 0; j < n_total && alive; j += 2, ++tile) {
-          alive = mbar_wait(bar(K_FULL + tile % KSTAGES), (tile / KSTAGES) & 1, abort_flag, spin_limit);
+          alive = mbar_wait_warp(bar(K_FULL + tile % KSTAGES), (tile / KSTAGES) & 1, abort_flag, spin_limit);
 #pragma unroll
           for (int x = 0; x < 2; ++x) {
             if (j >= w.n_tiles[x] || !alive) continue;
             const uint32_t u = n_s[x]++;
-            if (u > 0) alive = mbar_wait(bar(P_FULL + x), (u - 1) & 1, abort_flag, spin_limit);   // S has been read
-            alive = __all_sync(0xffffffffu, alive);
+            if (u > 0) alive = mbar_wait_warp(bar(P_FULL + x), (u - 1) & 1, abort_flag, spin_limit);   // S has been read
             if (!alive) break;
             tc_fence_after();
             if (elect_one()) {
@@ -424,7 +419,6 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
             }
             __syncwarp();
           }
-          alive = __all_sync(0xffffffffu, alive);
           if (!alive) break;
           if (elect_one()) {
             mma_commit(bar(K_EMPTY + tile % KSTAGES));
@@ -434,8 +428,7 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
         }
         continue;
       }
-      if (alive) alive = mbar_wait(bar(K_FULL + tile % KSTAGES), (tile / KSTAGES) & 1, abort_flag, spin_limit);
-      alive = __all_sync(0xffffffffu, alive);
+      if (alive) alive = mbar_wait_warp(bar(K_FULL + tile % KSTAGES), (tile / KSTAGES) & 1, abort_flag, spin_limit);
       if (!alive) break;
       tc_fence_after();
       if (elect_one()) {                               // S of both tiles is free: the last P has been waited for
@@ -454,12 +447,12 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
           const bool more = j + 1 < w.n_tiles[x];
           // the tiles this step reads normally landed long ago: check them before P, and only once per j
           if (x == 0 || j >= w.n_tiles[0]) {
-            alive = mbar_wait(bar(V_FULL + tile % VSTAGES), (tile / VSTAGES) & 1, abort_flag, spin_limit);
+            alive = mbar_wait_warp(bar(V_FULL + tile % VSTAGES), (tile / VSTAGES) & 1, abort_flag, spin_limit);
             if (alive && j + 1 < n_total)
-              alive = mbar_wait(bar(K_FULL + (tile + 1) % KSTAGES), ((tile + 1) / KSTAGES) & 1, abort_flag, spin_limit);
+              alive = mbar_wait_warp(bar(K_FULL + (tile + 1) % KSTAGES), ((tile + 1) / KSTAGES) & 1, abort_flag, spin_limit);
           }
           if (lane == 0) trace(2, j, x * 4 + 1);
-          if (alive) alive = mbar_wait(bar(P_FULL + x), (p_par >> x) & 1, abort_flag, spin_limit);
+          if (alive) alive = mbar_wait_warp(bar(P_FULL + x), (p_par >> x) & 1, abort_flag, spin_limit);
           if (!alive) break;
           p_par ^= 1u << x;
           tc_fence_after();
@@ -511,8 +504,8 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
       for (int j = 0; j < nx && alive; ++j) {
         if (r == 0) trace(x, j, 0);
         if (HAS_O || (j & 1) == 0) {                       // score-only: S of two tiles at a time
-          alive = __all_sync(0xffffffffu, mbar_wait(bar(S_FULL + x), s_par, abort_flag, spin_limit));
-          if (!alive) break;                               // the warp votes below: all of it goes on, or none
+          alive = mbar_wait_warp(bar(S_FULL + x), s_par, abort_flag, spin_limit);
+          if (!alive) break;
           s_par ^= 1;
         }
         const uint32_t tS = tmem + (HAS_O ? x * BN : x * 2 * BN + (j & 1) * BN) + lane_addr;
@@ -671,7 +664,7 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
 
       // ---- epilogue ----
       if (alive && nx > 0 && has_o) {
-        alive = __all_sync(0xffffffffu, mbar_wait(bar(O_FULL + x), o_par, abort_flag, spin_limit));
+        alive = mbar_wait_warp(bar(O_FULL + x), o_par, abort_flag, spin_limit);
         o_par ^= 1;
       }
       if (alive && has_o) {

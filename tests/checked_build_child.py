@@ -8,7 +8,8 @@ sources of the shipped library compiled with -DMSA_BOUNDS_CHECK -DMSA_DEBUG_HOOK
 3. A bounded wait that runs out: a test hook makes the TMA producer of the dense prefill kernel stop before its
    second K tile (issuing nothing after it) and shortens the poll limit.  The MMA warp's wait for that tile gives
    up, every role returns, TMEM is released, the status word says STATUS_TIMEOUT; while it is set the next launch
-   returns at once without touching its output; last_status() clears it and the kernel works again.
+   returns at once without touching its output; last_status() clears it and the kernel works again.  The same for
+   the score-only pass, whose MMA warp has waits of its own.
 Prints one line per part; exits non-zero on the first failure.
 """
 import ctypes
@@ -25,7 +26,7 @@ sys.path.insert(0, os.path.join(ROOT, "tests"))
 import msa_for_sail as msa                      # noqa: E402
 from msa_for_sail import _lib, api             # noqa: E402
 from oracle import msa_oracle as orc           # noqa: E402
-from helpers import check_out, gen, make_paged, randn_bf16, random_blocks   # noqa: E402
+from helpers import check_out, check_score, gen, make_paged, randn_bf16, random_blocks   # noqa: E402
 
 DEV = "cuda"
 assert _lib.BOUNDS_CHECK and _lib.LIB_PATH.endswith("libmsa_b200_check.so")
@@ -84,35 +85,47 @@ def part_bad_page():
     print("out-of-range page id: clamped, STATUS_BOUNDS reported and cleared")
 
 
-def part_timeout():
+def part_timeout(score_only):
     g = gen(3)
     qo, kv, hq, hk = [512], [512], 2, 1                   # 4 key tiles per CTA on the tcgen05 prefill kernel
     q = randn_bf16(g, 512, hq, 128); k = randn_bf16(g, 512, hk, 128); v = randn_bf16(g, 512, hk, 128)
-    plan = msa.fmha_sail_plan(i32(qo), i32(kv), hq, num_kv_heads=hk)
+    plan = msa.fmha_sail_plan(i32(qo), i32(kv), hq, num_kv_heads=hk, output_maxscore=score_only)
     assert plan[3]["tc_preferred"], "this shape is expected on the tcgen05 prefill kernel"
-    ref = orc.attention(q, k, v, qo, kv, hq, hk)
+    if score_only:
+        out = torch.empty(hq, plan[3]["max_k_tiles"], 512, device=DEV)
+        dest = dict(output_o=False, max_score=out)
+    else:
+        out = torch.empty(512, hq, 128, dtype=torch.bfloat16, device=DEV)
+        dest = dict(out=out)
+    run = lambda: msa.fmha_sail(q.to(DEV), k.to(DEV), v.to(DEV), plan, **dest)
+
     _lib.lib.msa_debug_tc_stall.argtypes = [ctypes.c_int, ctypes.c_uint]
     _lib.lib.msa_debug_tc_stall(1, 1 << 14)
-    out = torch.full((512, hq, 128), 7.0, dtype=torch.bfloat16, device=DEV)
-    msa.fmha_sail(q.to(DEV), k.to(DEV), v.to(DEV), plan, out=out)
+    out.fill_(7.0)
+    run()
     torch.cuda.synchronize()                               # returns: every wait in the kernel is bounded
     _lib.lib.msa_debug_tc_stall(-1, 0)
     st = api.last_status(reset=False)
     assert st == _lib.STATUS_TIMEOUT, f"expected STATUS_TIMEOUT, got {st}"
     out.fill_(7.0)
-    msa.fmha_sail(q.to(DEV), k.to(DEV), v.to(DEV), plan, out=out)     # status still set: CTAs return after their prologue
+    run()                                                  # status still set: CTAs return after their prologue
     torch.cuda.synchronize()
     assert (out == 7.0).all(), "a launch while the status word is set must not run"
     assert api.last_status() == _lib.STATUS_TIMEOUT and api.last_status() == 0
-    msa.fmha_sail(q.to(DEV), k.to(DEV), v.to(DEV), plan, out=out)
+    out.fill_(-float("inf") if score_only else 7.0)
+    run()
     torch.cuda.synchronize()
-    check_out(out, ref, "after the timeout was cleared")
+    if score_only:
+        check_score(out, orc.tile_max_score(q, k, qo, kv, hk, out.shape[1]), "after the timeout was cleared")
+    else:
+        check_out(out, orc.attention(q, k, v, qo, kv, hq, hk), "after the timeout was cleared")
     assert api.last_status() == 0
-    print("bounded wait ran out: STATUS_TIMEOUT, next launch skipped, cleared, kernel works again")
+    print("bounded wait ran out, score_only=%s: STATUS_TIMEOUT, next launch skipped, cleared, kernel works again" % score_only)
 
 
 if __name__ == "__main__":
     part_valid()
     part_bad_page()
-    part_timeout()
+    part_timeout(False)
+    part_timeout(True)
     print("CHECKED_BUILD_OK")

@@ -15,11 +15,12 @@ def code(name):
     return re.sub(r"//[^\n]*|/\*.*?\*/", "", text, flags=re.S)
 
 
-@pytest.mark.parametrize("name,begin,end", [("fmha_sparse_tc.cu", "const int gt =", "const uint64_t dk_hi")])
-def test_warps_wait_as_one(name, begin, end):
-    """A role of a tcgen05 kernel is one or more whole warps, each of which goes on as one: a bounded wait is voted on
-    (mbar_wait_warp).  The loaders of the sparse kernel: a lane that lagged could miss a phase for good."""
+@pytest.mark.parametrize("name", ["fmha_tc.cu", "fmha_sparse_tc.cu", "fmha_decode_tc.cu"])
+def test_warps_wait_as_one(name):
+    """A role of a tcgen05 kernel is one or more whole warps, each of which goes on as one: every bounded wait is voted on
+    (mbar_wait_warp).  A lane that lagged in a wait of its own could miss a phase for good; one that gave up alone would
+    leave the others in a warp-wide instruction."""
     text = code(name)
-    role = text[text.index(begin):text.index(end)]
-    assert "mbar_wait_warp(" in role
-    assert not re.search(r"\bmbar_wait\(", role)
+    assert "mbar_wait_warp(" in text
+    assert not re.search(r"\bmbar_wait\(", text)
+    assert not re.search(r"&& \*abort_flag", text)           # the other way out of a loop: read by each lane, decided by the warp
