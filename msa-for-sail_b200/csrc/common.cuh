@@ -37,6 +37,9 @@ __device__ __forceinline__ int chk(int v, int, int, int32_t*) { return v; }
 // until the kernel before has completed and its writes are visible (at once if there is nothing to wait for), then
 // lets the next kernel of the stream come up in the same way.  So the order of all memory accesses is that of the
 // stream, and only the launch and the start of the CTAs overlap.
+// What such a kernel reads may still be written while it starts, so it reads global memory with ordinary loads only: no
+// __ldg, ld.global.nc or __restrict__, which promise data that does not change during the kernel, and would allow a load
+// above the wait or a line of L1 from before it.
 __device__ __forceinline__ void chain_begin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -161,8 +161,8 @@ __device__ __forceinline__ bool entry_valid(const IndexArgs& a, int t, int b, in
 
 template <bool SCATTER>
 __global__ void __launch_bounds__(256)
-sparse_index_kernel(const IndexArgs a, int32_t* __restrict__ bin_count, int32_t* __restrict__ bin_cursor,
-                    int32_t* __restrict__ entries, int32_t* __restrict__ vmask) {
+sparse_index_kernel(const IndexArgs a, int32_t* bin_count, int32_t* bin_cursor,
+                    int32_t* entries, int32_t* vmask) {
   chain_begin();
   const int64_t gid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;   // kvh-major, token fastest
   const int64_t n = static_cast<int64_t>(a.total_q) * a.num_kv_heads;
@@ -190,8 +190,8 @@ sparse_index_kernel(const IndexArgs a, int32_t* __restrict__ bin_count, int32_t*
 // CTA.  Needs num_pages * 4 bytes of shared memory; larger page counts use the kernel above.
 template <bool SCATTER, int KBN>
 __global__ void __launch_bounds__(256)
-sparse_index_smem_kernel(const IndexArgs a, int32_t* __restrict__ bin_count, int32_t* __restrict__ bin_cursor,
-                         int32_t* __restrict__ entries, int32_t* __restrict__ vmask) {
+sparse_index_smem_kernel(const IndexArgs a, int32_t* bin_count, int32_t* bin_cursor,
+                         int32_t* entries, int32_t* vmask) {
   chain_begin();
   extern __shared__ int32_t s_hist[];                      // [num_pages] count, then (scatter) next position
   const int blocks_per_head = (a.total_q + 255) / 256;
@@ -241,8 +241,8 @@ sparse_index_smem_kernel(const IndexArgs a, int32_t* __restrict__ bin_count, int
 // per 1 024 bins; a scan in shared memory with a barrier pair per step made twenty-two (193 against 192 us a pass at 9 000
 // tokens, 1 620 against 1 593 us at 3 076 bins).
 __global__ void __launch_bounds__(1024)
-sparse_scan_kernel(const int32_t* __restrict__ bin_count, int32_t* __restrict__ bin_offset,
-                   int32_t* __restrict__ bin_cursor, int4* __restrict__ items, int32_t* __restrict__ part_start,
+sparse_scan_kernel(const int32_t* bin_count, int32_t* bin_offset,
+                   int32_t* bin_cursor, int4* items, int32_t* part_start,
                    int num_bins, int rows_per_item, int max_items, int tpc, int bins_per_head) {
   chain_begin();
   __shared__ int s_ent[32], s_itm[32];
@@ -306,8 +306,8 @@ struct MergeCfg {
 
 template <int KBN>
 __global__ void __launch_bounds__(MergeCfg<KBN>::WARPS * 32, 1)
-sparse_merge_kernel(const __nv_bfloat16* __restrict__ po, const float* __restrict__ pl, const int32_t* __restrict__ vmask,
-                    __nv_bfloat16* __restrict__ out, float* __restrict__ lse_out, int kbn, int n_rows, int num_heads,
+sparse_merge_kernel(const __nv_bfloat16* po, const float* pl, const int32_t* vmask,
+                    __nv_bfloat16* out, float* lse_out, int kbn, int n_rows, int num_heads,
                     int g_shift, int64_t out_stride_tok, int64_t out_stride_head, float out_scale) {
   chain_begin();
   using C = MergeCfg<KBN>;
@@ -317,7 +317,7 @@ sparse_merge_kernel(const __nv_bfloat16* __restrict__ po, const float* __restric
   const uint32_t mine_s = smem_u32(mine);
   const int G = 1 << g_shift;
   const int step = gridDim.x * C::WARPS * 2;
-  auto mask_of = [&](int row) -> uint32_t { return row < n_rows ? static_cast<uint32_t>(__ldg(vmask + (row >> g_shift))) : 0u; };
+  auto mask_of = [&](int row) -> uint32_t { return row < n_rows ? static_cast<uint32_t>(vmask[row >> g_shift]) : 0u; };
   auto prow_of = [&](int row) -> int64_t { return static_cast<int64_t>(row >> g_shift) * (kbn << g_shift) + (row & (G - 1)); };
   float lse[2][C::LPL];
   // request one row pair into a stage: the slots in `mask`, this lane's LSEs
@@ -332,7 +332,7 @@ sparse_merge_kernel(const __nv_bfloat16* __restrict__ po, const float* __restric
 #pragma unroll
     for (int i = 0; i < C::LPL; ++i) {
       const int s = l16 + 16 * i;
-      lse[stage][i] = (s < KBN && ((mask >> s) & 1u)) ? __ldg(pl + prow0 + (s << g_shift)) : -INFINITY;
+      lse[stage][i] = (s < KBN && ((mask >> s) & 1u)) ? pl[prow0 + (s << g_shift)] : -INFINITY;
     }
   };
   // combine one row pair out of a stage
@@ -404,9 +404,9 @@ template <bool F8>
 __global__ void __launch_bounds__(NTHREADS, 1)
 sparse_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ CUtensorMap tm_q,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-                 const int4* __restrict__ items, const int32_t* __restrict__ part_start, const int part,
-                 const int32_t* __restrict__ entries, float* __restrict__ partial_lse,
-                 __nv_bfloat16* __restrict__ partial_o) {
+                 const int4* items, const int32_t* part_start, const int part,
+                 const int32_t* entries, float* partial_lse,
+                 __nv_bfloat16* partial_o) {
   chain_begin();
   // this launch covers the work items of kv head `part`, or all of them (part < 0)
   const int item_idx = (part >= 0 ? part_start[part] : 0) + static_cast<int>(blockIdx.x);

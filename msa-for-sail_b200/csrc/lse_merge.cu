@@ -16,8 +16,8 @@ namespace {
 // eight splits are issued back to back before they are consumed.
 template <bool PBF16, bool OF32>
 __global__ void __launch_bounds__(256)
-lse_merge_kernel(const void* __restrict__ po_, const float* __restrict__ pl, const int32_t* __restrict__ spr,
-                 void* __restrict__ out_, float* __restrict__ lse_out, int num_splits, int total_q,
+lse_merge_kernel(const void* po_, const float* pl, const int32_t* spr,
+                 void* out_, float* lse_out, int num_splits, int total_q,
                  int num_heads, int64_t o_split_stride, int64_t l_split_stride, int64_t out_stride_tok,
                  int64_t out_stride_head, float out_scale) {
   chain_begin();
@@ -29,7 +29,7 @@ lse_merge_kernel(const void* __restrict__ po_, const float* __restrict__ pl, con
   const int S = spr ? min(spr[t], num_splits) : num_splits;
 
   float mx = -INFINITY;
-  for (int s = 0; s < S; ++s) mx = fmaxf(mx, __ldg(pl + static_cast<int64_t>(s) * l_split_stride + row));
+  for (int s = 0; s < S; ++s) mx = fmaxf(mx, pl[static_cast<int64_t>(s) * l_split_stride + row]);
   const float mxs = (mx == -INFINITY) ? 0.f : mx;
 
   float acc[8];
@@ -50,7 +50,7 @@ lse_merge_kernel(const void* __restrict__ po_, const float* __restrict__ pl, con
         raw[u][0] = *reinterpret_cast<const uint4*>(static_cast<const float*>(po_) + base);
         raw[u][1] = *reinterpret_cast<const uint4*>(static_cast<const float*>(po_) + base + 4);
       }
-      const float l = __ldg(pl + static_cast<int64_t>(s) * l_split_stride + row);
+      const float l = pl[static_cast<int64_t>(s) * l_split_stride + row];
       w[u] = (s0 + u < S && l != -INFINITY) ? __expf(l - mxs) : 0.f;
     }
 #pragma unroll

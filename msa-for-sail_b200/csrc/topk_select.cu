@@ -97,7 +97,7 @@ __device__ __forceinline__ void net_merge_desc(K (&key)[N], const K (&v)[N]) {
 // FORCED: some pages rank as FLT_MAX whatever their score.
 template <int TOPK, typename T, bool FORCED>
 __global__ void __launch_bounds__(512)
-topk_threshold_kernel(const T* __restrict__ scores, int32_t* __restrict__ out, int num_heads, int max_k_tiles,
+topk_threshold_kernel(const T* scores, int32_t* out, int num_heads, int max_k_tiles,
                       int total_q, int nvp, int force_begin, int force_end_start, int slices) {
   chain_begin();
   extern __shared__ uint32_t s_lists[];             // [slices][TOPK][32]: keys of the first scan, pages of the second
@@ -224,7 +224,7 @@ topk_threshold_kernel(const T* __restrict__ scores, int32_t* __restrict__ out, i
 
 template <int TOPK, typename T>
 __global__ void __launch_bounds__(256)
-topk_select_kernel(const T* __restrict__ scores, int32_t* __restrict__ out, int num_heads, int max_k_tiles,
+topk_select_kernel(const T* scores, int32_t* out, int num_heads, int max_k_tiles,
                    int total_q, int nvp, int slices) {
   chain_begin();
   using K = Key1;
@@ -330,7 +330,7 @@ __device__ __forceinline__ void warp_select_round(const uint32_t (&ord)[NKEYS], 
 
 template <int TOPK, int NK, typename T>
 __global__ void __launch_bounds__(256)
-topk_row_kernel(const T* __restrict__ scores, int32_t* __restrict__ out, int num_heads, int max_k_tiles, int total_q,
+topk_row_kernel(const T* scores, int32_t* out, int num_heads, int max_k_tiles, int total_q,
                 int nvp, int force_begin, int force_end_start) {
   chain_begin();
   static_assert(TOPK <= 32, "one winner per lane");
@@ -385,7 +385,7 @@ topk_row_kernel(const T* __restrict__ scores, int32_t* __restrict__ out, int num
 }
 
 template <int TOPK>
-__global__ void topk_identity_kernel(int32_t* __restrict__ out, size_t rows, int nvp) {
+__global__ void topk_identity_kernel(int32_t* out, size_t rows, int nvp) {
   chain_begin();
   const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= rows * TOPK) return;

@@ -222,3 +222,44 @@ def test_device_plan_prefix_sums(batch):
     for key, v in (("qo_segment_offsets", qo), ("kv_segment_offsets", kv), ("kv_page_indptr", -(-kv // 128))):
         assert plan[key].cpu().tolist() == [0] + np.cumsum(v).tolist(), key
     assert plan["qo_offset"].cpu().tolist() == (kv - qo).tolist()
+
+
+# ---- kernels of one stream that come up before the one before them has ended ----
+@pytest.mark.parametrize("tokens,kv", [(3, [2000, 700, 5000, 64]), (1100, [3000])])
+def test_chained_passes_read_the_latest_data(tokens, kv):
+    """Passes back to back into the same buffers, each on other inputs: bit for bit what a pass gives that nothing overlaps."""
+    import msa_for_sail as msa
+    g = torch.Generator(device=DEV).manual_seed(tokens)
+    hq, hk, topk, T = 16, 2, 4, tokens * len(kv)
+    P = sum(-(-n // 128) for n in kv)
+    nvp = -(-max(kv) // 128)
+    sets = [(torch.randn(T, hq, 128, device=DEV, generator=g).to(torch.bfloat16), torch.randn(T, hk, 128, device=DEV, generator=g).to(torch.bfloat16),
+             torch.randn(P, 1, 128, 128, device=DEV, generator=g).to(torch.bfloat16), torch.randn(P, hk, 128, 128, device=DEV, generator=g).to(torch.bfloat16),
+             torch.randn(P, hk, 128, 128, device=DEV, generator=g).to(torch.bfloat16)) for _ in range(3)]
+    buf = [torch.empty_like(t) for t in sets[0]]
+    q, iq, ik, k, v = buf
+    table = torch.randperm(P, device=DEV, generator=g).to(torch.int32)
+    lens = i32([tokens] * len(kv)), i32(kv)
+    score = msa.fmha_sail_plan(*lens, hk, num_kv_heads=1, page_size=128, output_maxscore=True)
+    sparse = msa.fmha_sail_plan(*lens, hq, num_kv_heads=hk, page_size=128, kv_block_num=topk, num_kv_splits=4)
+    scores = torch.full((hk, -(-nvp // 128) * 128, T), -float("inf"), device=DEV)
+    sel = torch.empty(T, hk, topk, dtype=torch.int32, device=DEV)
+
+    def one(i, sync):
+        for b, t in zip(buf, sets[i]):
+            b.copy_(t)
+        if sync:
+            torch.cuda.synchronize()
+        msa.fmha_sail(iq, ik, ik, score, kv_indices=table, output_o=False, max_score=scores)
+        if sync:
+            torch.cuda.synchronize()
+        msa.sparse_topk_select(scores, topk, num_valid_pages=nvp, output=sel)
+        if sync:
+            torch.cuda.synchronize()
+        return msa.fmha_sail(q, k, v, sparse, kv_indices=table, kv_block_indexes=sel)[0]
+
+    want = [one(i, True) for i in range(3)]
+    assert not torch.equal(want[0], want[1])
+    got = [one(i % 3, False) for i in range(60)]
+    for i, out in enumerate(got):
+        assert torch.equal(out, want[i % 3]), i

@@ -24,3 +24,15 @@ def test_warps_wait_as_one(name):
     assert "mbar_wait_warp(" in text
     assert not re.search(r"\bmbar_wait\(", text)
     assert not re.search(r"&& \*abort_flag", text)           # the other way out of a loop: read by each lane, decided by the warp
+
+
+@pytest.mark.parametrize("name", sorted(n for n in os.listdir(CSRC) if n.endswith(".cu")))
+def test_chained_kernels_wait_and_read_coherently(name):
+    """A kernel launched with launch_chained() is up while the one before it still writes: it waits with chain_begin(), and
+    reads global memory in no way that takes the data to be constant during the kernel."""
+    text = code(name)
+    kernels = text.split("__global__")[1:]
+    if "launch_chained(" in text:
+        assert kernels and all("chain_begin();" in k for k in kernels)
+        for k in kernels:
+            assert not re.search(r"__restrict__|__ldg\b|\.nc\b", k)
