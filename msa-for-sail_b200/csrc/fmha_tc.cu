@@ -173,14 +173,19 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  // item number `it` of this CTA, for a whole warp: false when there is none or a wait of any lane gave up
-  auto take_item = [&](uint32_t it, Item& w, bool alive) -> bool {
+  // Item number `it` of this CTA, for a whole warp: false when there is none or a wait of any lane gave up.  The warp may
+  // come here early, since a Q tile without rows or visible keys has no work, and then waits for the other warps to get to
+  // the end of the item before, of `tiles` KV tiles (0 at first): the one wait, with the scheduler's, that may last as long
+  // as an item, so its limit grows with it.  (The roles that it waits for are bounded tile by tile and raise the abort flag.)
+  auto item_limit = [&](int tiles) -> uint64_t { return static_cast<uint64_t>(spin_limit) * (1u + static_cast<uint32_t>(tiles)); };
+  auto take_item = [&](uint32_t it, Item& w, int& tiles, bool alive) -> bool {
     if (!alive) return false;
     const uint32_t slot = it & 1;
-    if (!mbar_wait_warp(bar(ITEM_FULL + slot), (it >> 1) & 1, abort_flag, spin_limit)) return false;
+    if (!mbar_wait_warp(bar(ITEM_FULL + slot), (it >> 1) & 1, abort_flag, item_limit(tiles))) return false;
     w = items[slot];
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(ITEM_EMPTY + slot));
+    tiles = max(w.n_tiles[0], w.n_tiles[1]);
     return w.valid != 0;
   };
 
@@ -194,8 +199,9 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
     uint32_t fix_phase = 0, tile = 0, q_loads = 0;      // running counts: the rings go on from item to item
     bool alive = true;
     Item w;
-    for (uint32_t it = 0; take_item(it, w, alive); ++it) {
-      const int n_total = max(w.n_tiles[0], w.n_tiles[1]), head = w.head, kvh = w.kvh, kv_len = w.kv_len;
+    int n_total = 0;
+    for (uint32_t it = 0; take_item(it, w, n_total, alive); ++it) {
+      const int head = w.head, kvh = w.kvh, kv_len = w.kv_len;
       const int page_base = w.kv0, kv_base = w.kv0;
       if (n_total > 0) {                                  // an item without visible keys loads nothing
         alive = mbar_wait_warp(bar(Q_EMPTY), (q_loads & 1) ^ 1, abort_flag, spin_limit);
@@ -337,7 +343,7 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
       }
       __syncwarp();
       if (idx < 0) break;
-      alive = mbar_wait_warp(bar(NEXT_REQ), it & 1, abort_flag, spin_limit);
+      alive = mbar_wait_warp(bar(NEXT_REQ), it & 1, abort_flag, item_limit(max(w.n_tiles[0], w.n_tiles[1])));
       if (!alive) break;
       if (lane == 0) {
         mbar_arrive_expect_tx(bar(NEXT_FULL), 16);
@@ -390,8 +396,8 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
     [[maybe_unused]] uint32_t n_s[2] = {0, 0};         // score-only: S pairs issued so far
     bool alive = true;
     Item w;
-    for (uint32_t it = 0; take_item(it, w, alive); ++it) {
-      const int n_total = max(w.n_tiles[0], w.n_tiles[1]);
+    int n_total = 0;
+    for (uint32_t it = 0; take_item(it, w, n_total, alive); ++it) {
       if (n_total == 0) continue;
       alive = mbar_wait_warp(bar(Q_FULL), q_loads & 1, abort_flag, spin_limit);
       ++q_loads;
@@ -489,7 +495,8 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
     bool alive = true;
     uint32_t s_par = 0, o_par = 0;
     Item w;
-    for (uint32_t it = 0; take_item(it, w, alive); ++it) {
+    int n_total = 0;
+    for (uint32_t it = 0; take_item(it, w, n_total, alive); ++it) {
       const int head = w.head, kvh = w.kvh, kv_len = w.kv_len, off = w.off;
       const int m0 = w.row0 + x * BM;
       const int i = m0 + r;                                // token index within the sequence

@@ -50,9 +50,10 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
 // Bounded wait: gives up after kSpinLimit polls or as soon as another thread of the CTA has
 // raised the abort flag; returns false in that case (and raises the flag itself).
 constexpr uint32_t kSpinLimit = 1u << 21;
+template <typename Count = uint32_t>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          uint32_t limit = kSpinLimit) {
-  for (uint32_t i = 0; i < limit; ++i) {
+                                          Count limit = kSpinLimit) {
+  for (Count i = 0; i < limit; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((i & 1023u) == 1023u && *abort_flag) return false;
   }
@@ -62,8 +63,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 // The wait of a warp that goes on as one: every lane has seen the phase, or none goes on.  A lane on its own could lag
 // behind its neighbours until the phase it waits for has come and gone (two phases of a barrier look alike), or give up
 // where they went on, and leave them in a warp-wide instruction.
+template <typename Count = uint32_t>
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                               uint32_t limit = kSpinLimit) {
+                                               Count limit = kSpinLimit) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, limit));
 }
 

@@ -10,6 +10,9 @@ sources of the shipped library compiled with -DMSA_BOUNDS_CHECK -DMSA_DEBUG_HOOK
    up, every role returns, TMEM is released, the status word says STATUS_TIMEOUT; while it is set the next launch
    returns at once without touching its output; last_status() clears it and the kernel works again.  The same for
    the score-only pass, whose MMA warp has waits of its own.
+4. Waits that last as long as a work item: with a limit that is ample for a tile (4 096 polls) and far too short for
+   an item of 8 192 tiles (10 ms and more), nothing gives up -- neither the scheduler, which waits for the end of the
+   item, nor the softmax warps of a Q tile that has no rows.
 Prints one line per part; exits non-zero on the first failure.
 """
 import ctypes
@@ -123,9 +126,35 @@ def part_timeout(score_only):
     print("bounded wait ran out, score_only=%s: STATUS_TIMEOUT, next launch skipped, cleared, kernel works again" % score_only)
 
 
+def part_long_item():
+    g = torch.Generator(device=DEV).manual_seed(4)
+    n, rows = 1 << 20, 384                                 # items of 256 rows and of 128 (no second Q tile)
+    q, k, v = (torch.randn(m, 1, 128, device=DEV, generator=g, dtype=torch.bfloat16) for m in (rows, n, n))
+    q *= 4                                                 # so that the result is more than the mean of V
+    s = (q[:, 0].float() @ k[:, 0].float().T) * 128 ** -0.5
+    hidden = torch.arange(n, device=DEV)[None, :] > torch.arange(n - rows, n, device=DEV)[:, None]
+    s.masked_fill_(hidden, -float("inf"))
+    ref = torch.softmax(s, 1) @ v[:, 0].float()
+    tiles = s.view(rows, n // 128, 128).amax(-1).T / 128 ** -0.5
+    _lib.lib.msa_debug_tc_stall(-1, 1 << 12)
+    for score_only in (False, True):
+        plan = msa.fmha_sail_plan(i32([rows]), i32([n]), 1, num_kv_heads=1, num_kv_splits=1, output_maxscore=score_only)
+        assert plan[3]["tc_preferred"]
+        out, ms = msa.fmha_sail(q, k, v, plan, output_o=not score_only)
+        torch.cuda.synchronize()
+        assert api.last_status() == 0, "a wait for a whole item gave up"
+        if score_only:
+            check_score(ms[0], tiles.cpu(), "long item")
+        else:
+            check_out(out[:, 0], ref.cpu(), "long item")
+    _lib.lib.msa_debug_tc_stall(-1, 0)
+    print("items of 8 192 tiles with 4 096 polls a tile: ok, status 0")
+
+
 if __name__ == "__main__":
     part_valid()
     part_bad_page()
     part_timeout(False)
     part_timeout(True)
+    part_long_item()
     print("CHECKED_BUILD_OK")
