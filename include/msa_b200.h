@@ -179,7 +179,8 @@ typedef struct MsaPlanArgs {
   int32_t pack;               /* 1 or Hq/Hkv   */
   int32_t num_splits;         /* >=1 fixed; <=0 adaptive with -num_splits as the ceiling */
   int32_t num_sms;            /* device SM count (adaptive mode target)  */
-  int32_t ctas_per_sm;        /* items an SM runs side by side; 0 = 1 (adaptive mode) */
+  int32_t ctas_per_sm;        /* items an SM runs side by side; 0 = 1; < 0: all items cut alike, for two waves of the
+                               * SMs, and uncut where there are as many (adaptive mode) */
 } MsaPlanArgs;
 int msa_plan_dense(const MsaPlanArgs* args, MsaWorkItem* work, int32_t capacity,
                    int32_t* splits_per_row /* [total_q] host */,

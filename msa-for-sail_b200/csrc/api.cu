@@ -151,19 +151,22 @@ extern "C" int msa_plan_dense(const MsaPlanArgs* a, MsaWorkItem* work, int32_t c
     // Decode: one row tile per batch item.  Cutting the items at just above the average load of an SM gives nearly every
     // SM one full piece and leaves the remainders to fill up the rest; whichever of the two cuts ends earlier is taken.
     // (Ragged lengths are where it pays: 31 sequences of 515 to 7 001 keys x 4 heads: 28 tile times against 40.)
-    if (max_tiles > 4 && static_cast<int>(protos.size()) <= a->batch && items < 8LL * sms) {
+    if (a->ctas_per_sm >= 0 && max_tiles > 4 && static_cast<int>(protos.size()) <= a->batch && items < 8LL * sms) {
       const int slots = sms * std::max(1, a->ctas_per_sm);
       long long total = 0;
       for (const Proto& pr : protos) total += static_cast<long long>(pr.ntiles) * groups;
       int cut = std::max(4, static_cast<int>((total * 103 + 100LL * slots - 1) / (100LL * slots)));
-      // no more splits than the ceiling, nor than the library's own scratch holds where the plain cut fits it
+      // No more splits than the ceiling, nor than the library's own scratch holds where the plain cut fits it.  Every row
+      // has as many partial rows as the longest item has splits, so one long sequence among many short ones would ask for
+      // gigabytes: the partials take no more rows than those of a plain cut can (fewer than 2 x SMs items of block_m rows,
+      // cut into 2 x SMs pieces or up to twice that), or what this batch's plain cut takes.
       long long rows = 0;
       for (int b = 0; b < a->batch; ++b) rows += static_cast<long long>(a->qo_len[b]) * a->num_qo_heads;
+      rows = std::max(1LL, rows);
       const int plain_splits = (max_tiles + chunk - 1) / chunk;
-      int most = ceiling;
-      if (plain_splits * rows <= MSA_STATIC_SCRATCH_MAX_ROWS)
-        most = static_cast<int>(std::min<long long>(most, MSA_STATIC_SCRATCH_MAX_ROWS / std::max(1LL, rows)));
-      cut = std::max(cut, (max_tiles + most - 1) / most);
+      long long most = std::min<long long>(ceiling, std::max<long long>(plain_splits, 4LL * sms * a->block_m / rows));
+      if (plain_splits * rows <= MSA_STATIC_SCRATCH_MAX_ROWS) most = std::min(most, MSA_STATIC_SCRATCH_MAX_ROWS / rows);
+      cut = std::max(cut, static_cast<int>((max_tiles + most - 1) / most));
       if (cut < max_tiles && msa::makespan(protos, groups, cut, slots) < msa::makespan(protos, groups, chunk, slots)) chunk = cut;
     }
   }

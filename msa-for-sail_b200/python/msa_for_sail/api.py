@@ -164,6 +164,13 @@ class _Arena:
         self.off = end
         return out
 
+    def fits(self, sizes):
+        """Whether arrays of so many 4-byte elements, taken in this order, fit."""
+        end = self.off
+        for n in sizes:
+            end = ((end + 255) & ~255) + 4 * n
+        return self.buf is None or end <= self.buf.numel()
+
 
 class _Upload:
     """The int32 arrays of one plan, laid out in one block (256 bytes apart) and copied to the device at once: a copy
@@ -364,32 +371,9 @@ def _fmha_sail_plan(
                                        and total_q * kv_block_num >= 8 * info["num_logical_pages"])
     else:
         info["token_batch"] = None
-        args = _lib.MsaPlanArgs(
-            a_q.ctypes.data, a_k.ctypes.data, a_o.ctypes.data, batch, num_qo_heads, hkv, block_m, pack,
-            num_kv_splits if num_kv_splits >= 1 else -128, num_sms,
-            2 if use_fp8_kvcache and max_qo * pack <= 16 else 1)      # two CTAs of the e4m3 decode kernel share an SM
-        cap = 1024
-        spr = np.ones(max(1, total_q), np.int32)
-        max_splits = _lib._i32(1)
-        while True:
-            host = np.empty((cap, 8), np.int32)
-            n = _lib.lib.msa_plan_dense(ctypes.byref(args), host.ctypes.data, cap, spr.ctypes.data,
-                                        ctypes.byref(max_splits))
-            if n == -4:
-                cap *= 4
-                continue
-            _lib.check(n, "msa_plan_dense")
-            break
-        num_work = n
-        splits = int(max_splits.value)
-        up.add("work", host[:n], max(1, n) * 8)
-        info["_work_host"] = host[:n]
-        if splits > 1:
-            up.add("num_kv_splits_per_row", spr[:total_q])
         # second work list in 256-row items for the tcgen05 prefill kernel (q and k both bf16 or
         # both e4m3, unsplit, one query head per row tile, ragged K/V or 128-key pages)
         info["work_tc"], info["num_work_tc"] = None, 0
-        info["tc_preferred"] = False
         if pack == 1 and max_qo > 128 and page_size in (-1, 0, 128):
             args_tc = _lib.MsaPlanArgs(
                 a_q.ctypes.data, a_k.ctypes.data, a_o.ctypes.data, batch, num_qo_heads, hkv, 256, 1,
@@ -401,9 +385,36 @@ def _fmha_sail_plan(
             if n_tc:
                 up.add("work_tc", host_tc[:n_tc])
                 info["num_work_tc"] = n_tc
-                # with far too few items to fill the GPU the split-KV plan of the generic kernel wins
-                # (a 256-row tcgen05 item runs about three times as fast as the same rows there)
-                info["tc_preferred"] = splits == 1 or n_tc * 2 >= num_sms
+        # Two CTAs of the e4m3 decode kernel share an SM.  A cut at the average load may take more partials than a workspace
+        # sized for the plain cut holds: such a workspace gets the plain cut.
+        for ctas in (2 if use_fp8_kvcache and max_qo * pack <= 16 else 1, -1):
+            args = _lib.MsaPlanArgs(
+                a_q.ctypes.data, a_k.ctypes.data, a_o.ctypes.data, batch, num_qo_heads, hkv, block_m, pack,
+                num_kv_splits if num_kv_splits >= 1 else -128, num_sms, ctas)
+            cap = 1024
+            spr = np.ones(max(1, total_q), np.int32)
+            max_splits = _lib._i32(1)
+            while True:
+                host = np.empty((cap, 8), np.int32)
+                n = _lib.lib.msa_plan_dense(ctypes.byref(args), host.ctypes.data, cap, spr.ctypes.data,
+                                            ctypes.byref(max_splits))
+                if n == -4:
+                    cap *= 4
+                    continue
+                _lib.check(n, "msa_plan_dense")
+                break
+            num_work = n
+            splits = int(max_splits.value)
+            rows = splits * total_q * orig_num_qo_heads
+            if splits == 1 or arena.fits([size for *_, size in up.parts] + [max(1, n) * 8, total_q, rows * 128, rows]):
+                break
+        up.add("work", host[:n], max(1, n) * 8)
+        info["_work_host"] = host[:n]
+        if splits > 1:
+            up.add("num_kv_splits_per_row", spr[:total_q])
+        # with far too few items to fill the GPU the split-KV plan of the generic kernel wins
+        # (a 256-row tcgen05 item runs about three times as fast as the same rows there)
+        info["tc_preferred"] = info["num_work_tc"] > 0 and (splits == 1 or info["num_work_tc"] * 2 >= num_sms)
 
     up.run(arena, info)
     if splits > 1:

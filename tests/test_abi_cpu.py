@@ -252,3 +252,57 @@ def test_shipped_library_exports_no_debug_hooks():
     names = {ln.split()[-1] for ln in out.splitlines() if ln.strip()}
     assert not [n for n in names if n.startswith("msa_debug")], names
     assert set(L.EXPORTS) <= names
+
+
+def _host_plan(monkeypatch, qo, kv, hq, hk, **kw):
+    """A plan made on the host as the public entry point makes it, its arrays in CPU tensors."""
+    import torch
+    from msa_for_sail import api
+    monkeypatch.setattr(api, "_num_sms", lambda dev: 148)
+    as_i32 = lambda v: torch.tensor(v, dtype=torch.int32)
+    return api._fmha_sail_plan(as_i32(qo), as_i32(kv), hq, hk, page_size=128, device="cpu", **kw)
+
+
+@pytest.mark.parametrize("qo,kv,hq,hk,bm", [
+    ([4] * 300, [500] * 299 + [1 << 20], 16, 1, 64),
+    ([8] * 300, [500] * 299 + [1 << 20], 16, 1, 128),
+    ([16] * 64, [1000] * 63 + [131072], 64, 8, 128),
+    ([1] * 40, list(range(500, 39500, 1000)) + [100000], 64, 8, 16),
+    ([1] * 1100, [300] * 1099 + [200000], 8, 1, 16),
+])
+def test_adaptive_cut_bounds_its_partials(qo, kv, hq, hk, bm):
+    """Every row has as many partial rows as the longest item has splits: one long sequence among many short ones must
+    not ask for more of them than a plain cut of any batch does."""
+    L = _lib()
+    work, spr, splits = _plan(L, qo, kv, [k - q for q, k in zip(qo, kv)], hq, hk, bm, hq // hk, -128)
+    assert splits == 1 or splits * sum(qo) * hq <= 4 * 148 * bm
+    assert splits == 1 or len(qo) * hk < 8 * 148
+
+
+@pytest.mark.parametrize("qo,kv,hq,hk", [
+    ([1] * 100, [1000] * 99 + [131072], 32, 4),            # as many items as two waves: uncut by the plain rule
+    ([1] * 40, list(range(500, 39500, 1000)) + [100000], 64, 8),
+])
+def test_plan_goes_into_a_workspace_for_one_split(monkeypatch, qo, kv, hq, hk):
+    """Both defaults together, a workspace for one split and adaptive splits: the plan is uncut where the plain rule does not
+    cut; a larger workspace and none at all get the finer cut."""
+    import torch
+    from msa_for_sail import api
+    need = api._workspace_bytes(len(qo), sum(qo), hq, 1, False)
+    plan = _host_plan(monkeypatch, qo, kv, hq, hk, given_workspace=torch.empty(need, dtype=torch.uint8))
+    assert plan["num_kv_splits"] == 1 and plan["num_work"] == len(qo) * hk and plan["workspace_o"] is None
+    free = _host_plan(monkeypatch, qo, kv, hq, hk)
+    assert free["num_kv_splits"] > 1
+    ample = torch.empty(need + free["num_kv_splits"] * sum(qo) * hq * 640 + 100000, dtype=torch.uint8)
+    given = _host_plan(monkeypatch, qo, kv, hq, hk, given_workspace=ample)
+    assert given["num_kv_splits"] == free["num_kv_splits"] and torch.equal(given["work"], free["work"])
+    # exactly what the finer cut takes, and one element less
+    end = given["workspace_lse"].data_ptr() + given["workspace_lse"].numel() * 4 - ample.data_ptr()
+    assert _host_plan(monkeypatch, qo, kv, hq, hk, given_workspace=ample[:end])["num_kv_splits"] == free["num_kv_splits"]
+    assert _host_plan(monkeypatch, qo, kv, hq, hk, given_workspace=ample[:end - 4])["num_kv_splits"] == 1
+
+
+def test_plan_refuses_a_workspace_that_is_too_small(monkeypatch):
+    import torch
+    with pytest.raises(ValueError, match="too small"):
+        _host_plan(monkeypatch, [1] * 3, [9000, 5000, 100], 32, 4, given_workspace=torch.empty(100000, dtype=torch.uint8))
