@@ -115,14 +115,23 @@ def _compute_pack_factor(max_qo_len, num_qo_heads, num_kv_heads):
     return h_r
 
 
-def _sparse_splits(items, kv_block_num, most, num_sms, two_per_sm):
-    """Splits of the selected pages in token-major sparse attention: `most`, halved as often as pays.  A CTA takes its
+def _sparse_splits(items, kv_block_num, num_kv_splits, num_sms, two_per_sm):
+    """Splits of the selected pages in token-major sparse attention, halved as often as pays.  A CTA takes its
     pages and about four page times more (dependent index loads, the first page's latency, the epilogue), the CTAs run in
     rounds of the slots there are (two e4m3 CTAs of at most 16 rows share an SM), and splits cost a merge, about four
     page times.  24 tokens x 4 heads x 16 bf16 pages: 192 CTAs of 8 pages and the merge 36 us, 96 of 16 pages 26 us."""
+    # The most splits, which partials in a caller's workspace are sized for: enough CTAs for two rounds, or of an explicit
+    # count what is left once halving it would leave an SM without a CTA.
+    if num_kv_splits >= 1:
+        s = min(num_kv_splits, kv_block_num)
+        while s > 1 and items * (s // 2) >= num_sms:
+            s //= 2
+    else:
+        s = 1
+        while s * 2 <= min(kv_block_num, 8) and items * s < 2 * num_sms:
+            s *= 2
     slots = num_sms * (2 if two_per_sm else 1)
     best, best_cost = 1, None
-    s = min(most, kv_block_num)
     while s >= 1:
         cost = -(-items * s // slots) * (-(-kv_block_num // s) + 4) + (4 if s > 1 else 0)
         if best_cost is None or cost <= best_cost:
@@ -360,7 +369,7 @@ def _fmha_sail_plan(
     num_work = 0
     info["work"] = info["num_kv_splits_per_row"] = None
     if is_sparse:
-        splits = _sparse_splits(total_q * hkv, kv_block_num, num_kv_splits if num_kv_splits >= 1 else 8, num_sms,
+        splits = _sparse_splits(total_q * hkv, kv_block_num, num_kv_splits, num_sms,
                                 use_fp8_kvcache and h_r <= 16)
         up.add("token_batch", np.repeat(np.arange(batch, dtype=np.int32), a_q))
         up.add("page_batch", np.repeat(np.arange(batch, dtype=np.int32), pages_per))

@@ -306,3 +306,28 @@ def test_plan_refuses_a_workspace_that_is_too_small(monkeypatch):
     import torch
     with pytest.raises(ValueError, match="too small"):
         _host_plan(monkeypatch, [1] * 3, [9000, 5000, 100], 32, 4, given_workspace=torch.empty(100000, dtype=torch.uint8))
+
+
+@pytest.mark.parametrize("items", [1, 7, 64, 147, 148, 200, 296, 297, 330, 370, 371, 1024])
+@pytest.mark.parametrize("topk", [4, 8, 16, 32])
+def test_sparse_splits_fit_what_they_were_sized_for(monkeypatch, items, topk):
+    """Splits of the selected pages: never more than give two CTAs to every SM, or than an explicit count leaves of itself
+    once the items fill the SMs; so a workspace for one split takes any batch that needs no more."""
+    import torch
+    from msa_for_sail import api
+    plain = 1
+    while plain * 2 <= min(topk, 8) and items * plain < 296:
+        plain *= 2
+    plan = _host_plan(monkeypatch, [1] * items, [128 * topk] * items, 8, 1, kv_block_num=topk)
+    assert 1 <= plan["num_kv_splits"] <= plain
+    if plain == 1:
+        need = api._workspace_bytes(items, items, 8, 1, True) + items * topk * 4
+        given = _host_plan(monkeypatch, [1] * items, [128 * topk] * items, 8, 1, kv_block_num=topk,
+                           given_workspace=torch.empty(need, dtype=torch.uint8))
+        assert given["num_kv_splits"] == 1
+    for n in (1, 2, 4, 32):
+        plain = min(n, topk)
+        while plain > 1 and items * (plain // 2) >= 148:
+            plain //= 2
+        plan = _host_plan(monkeypatch, [1] * items, [128 * topk] * items, 8, 1, kv_block_num=topk, num_kv_splits=n)
+        assert plan["num_kv_splits"] <= plain
