@@ -73,6 +73,21 @@ constexpr int REGS_SOFTMAX = 152, REGS_OTHER = 40;
 constexpr int REGS_NEEDED = NWG * 128 * REGS_SOFTMAX + (GATHER_WARPS + 1) * 32 * REGS_OTHER;
 static_assert(NTHREADS == (MMA_WARP + 1) * 32, "warp roles");
 static_assert(REGS_NEEDED <= 65536, "setmaxnreg budget");
+// The Q boxes of a chunk are dealt out unit by unit: unit n (8 rows of a token, or a whole token where a group has fewer than 8
+// heads) to loader warp n % 3.  `upt`: units of a token.  Whether a loader warp has a unit in a chunk of `ntok` tokens:
+constexpr bool loader_has_unit(int loader, int upt, int ntok) { return loader / upt < ntok; }
+constexpr bool loader_has_unit_agrees() {                  // with the dealing itself, for every group size and chunk
+  for (int G = 1; G <= BM; G *= 2)
+    for (int ntok = 1; ntok <= BM / G; ++ntok)
+      for (int loader = 0; loader < GATHER_WARPS; ++loader) {
+        const int upt = G >= 8 ? G / 8 : 1;
+        bool any = false;
+        for (int unit = loader; unit < ntok * upt; unit += GATHER_WARPS) any = true;
+        if (any != loader_has_unit(loader, upt, ntok)) return false;
+      }
+  return true;
+}
+static_assert(loader_has_unit_agrees(), "a loader leaves before the wait for a chunk exactly where it has no unit in it");
 // Chunks of 128 rows per work item: a list of one page in pieces of 32, of 16 where an SM gets fewer than 128 chunks in
 // all and the last round weighs more than the pages loaded twice (9 000 tokens x 16 heads x 8 pages: 193 us a pass
 // against 198; 8: 205.  65 536 chunks: 1 654 us with 16, 1 620 with 32; 524 288 chunks: 32, 64 and 128 within 1 %).
@@ -532,7 +547,7 @@ sparse_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
       // A warp without a row in the (last, partial) chunk must not wait for its buffer: Q K^T of that chunk does not need
       // the warp and may give the buffer back first, and the parity the warp waits for would then never come.  The first
       // warp always has a row, and announces the chunk's bytes.
-      if ((warp - GATHER_WARP0) / upt >= min(tpc, item.z - (item.y + c * tpc))) break;
+      if (!loader_has_unit(warp - GATHER_WARP0, upt, min(tpc, item.z - (item.y + c * tpc)))) break;
       if (gt == 0) trace(4, c, 0);
       // Q K^T of chunk c - NQBUF has read the buffer.  The same holds for a lane as for a warp: most lanes have no unit, and
       // none may still wait here when the others' rows let Q K^T of this chunk turn the phase.

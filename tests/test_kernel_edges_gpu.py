@@ -173,27 +173,23 @@ def test_sparse_merge_edges(kbn, hq, hk, T):
     assert (lse - ref_lse)[seen].abs().max() <= 2e-3
 
 
-@pytest.mark.parametrize("dtype,hq,hk", [(torch.float8_e4m3fn, 16, 1), (torch.bfloat16, 8, 1)])
-def test_sparse_prefill_partial_chunks(dtype, hq, hk):
+@pytest.mark.parametrize("dtype", [torch.float8_e4m3fn, torch.bfloat16])
+def test_sparse_prefill_partial_chunks(dtype):
     """Page lists whose last chunk has one token, so that two of the three loader warps have no row in it: a loader that
     waited for that chunk's buffer all the same could miss its phase and run into the limit of its wait."""
     import msa_for_sail as msa
     from msa_for_sail import api
     g = gen(77)
-    pages, tpc = 64, 128 * hk // hq
-    # every page is selected by the same number of tokens: one more than a multiple of a chunk's
+    hq, hk, pages, topk = 8, 1, 64, 4
+    tpc = 128 * hk // hq                                     # a token is one unit: the last chunk has one
     per_page = 5 * tpc + 1
-    T = pages * per_page // 4
+    # 16 tokens after another share out all 64 pages, so that each page is selected equally often
+    bi = torch.cat([torch.randperm(pages, generator=g).view(pages // topk, topk) for _ in range(per_page)])
+    T = bi.shape[0]
     kv = [pages * 128 + T]
-    order = torch.randperm(pages * per_page, generator=g)[:T * 4] % pages
-    bi = order.view(T, 4)
-    for c in range(1, 4):                                    # four different pages a token
-        while True:
-            clash = (bi[:, :c] == bi[:, c:c + 1]).any(1)
-            if not clash.any():
-                break
-            bi[clash, c] = (bi[clash, c] + 1) % pages
-    bi = bi.sort(1).values.to(torch.int32).view(T, 1, 4)
+    assert (torch.bincount(bi.view(-1), minlength=pages) == per_page).all() and per_page % tpc == 1
+    bi = bi.sort(1).values.to(torch.int32).view(T, hk, topk)
+    assert (bi[:, :, 1:] > bi[:, :, :-1]).all()
     q = randn_bf16(g, T, hq, 128).to(dtype).to(DEV)
     kp, vp, table = make_paged(g, kv, hk, 128, dtype=dtype)
     kp, vp, table, bi = kp.to(DEV), vp.to(DEV), table.to(DEV), bi.to(DEV)

@@ -26,6 +26,14 @@ def test_warps_wait_as_one(name):
     assert not re.search(r"&& \*abort_flag", text)           # the other way out of a loop: read by each lane, decided by the warp
 
 
+def test_sparse_loader_leaves_before_the_wait():
+    """A loader warp without a unit in the last chunk of a list may not wait for that chunk's buffer (the phase it waits for
+    can be over by then).  That the condition is right for every group size and chunk is asserted when the file is compiled."""
+    loop = code("fmha_sparse_tc.cu").split("int ent = entry_of(0);")[1]
+    leave = loop.index("if (!loader_has_unit(warp - GATHER_WARP0, upt, min(tpc, item.z - (item.y + c * tpc)))) break;")
+    assert leave < loop.index("mbar_wait")
+
+
 @pytest.mark.parametrize("name", sorted(n for n in os.listdir(CSRC) if n.endswith(".cu")))
 def test_chained_kernels_wait_and_read_coherently(name):
     """A kernel launched with launch_chained() is up while the one before it still writes: it waits with chain_begin(), and
