@@ -780,7 +780,10 @@ decode_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant_
   // ---------------- teardown ----------------
   tc_fence_before();
   __syncthreads();
-  if (*abort_flag && threadIdx.x == 0 && p.status) atomicExch(p.status, MSA_STATUS_TIMEOUT);
+  if (*abort_flag) {
+    if (threadIdx.x == 0 && p.status) atomicExch(p.status, MSA_STATUS_TIMEOUT);
+    outlast_async_work();
+  }
 #ifdef MSA_DEBUG_HOOKS
   if (trace) { trace[13] = clock64() - clk0; trace[1] = global_ns(); }
 #endif

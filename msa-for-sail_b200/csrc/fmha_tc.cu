@@ -713,7 +713,10 @@ fmha_tc_kernel(const __grid_constant__ MsaFmhaParams p, const __grid_constant__ 
   // ---------------- teardown ----------------
   tc_fence_before();
   __syncthreads();
-  if (*abort_flag && threadIdx.x == 0 && p.status) atomicExch(p.status, MSA_STATUS_TIMEOUT);
+  if (*abort_flag) {
+    if (threadIdx.x == 0 && p.status) atomicExch(p.status, MSA_STATUS_TIMEOUT);
+    outlast_async_work();
+  }
   if (warp == MMA_WARP) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);

@@ -69,6 +69,13 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, limit));
 }
 
+// Once a wait has given up, copies and MMAs that the CTA issued may still be on their way into its shared memory and TMEM, and
+// which ones is no longer known.  They take microseconds: the CTA stays for a millisecond or so before it gives both back.
+__device__ __forceinline__ void outlast_async_work() {
+  const long long start = clock64();
+  for (int i = 0; i < 4096 && clock64() - start < 2000000; ++i) __nanosleep(1000);
+}
+
 // One lane of a converged warp (the compiler can keep the operands of the instructions issued
 // under this predicate in uniform registers).
 __device__ __forceinline__ bool elect_one() {

@@ -26,6 +26,13 @@ def test_warps_wait_as_one(name):
     assert not re.search(r"&& \*abort_flag", text)           # the other way out of a loop: read by each lane, decided by the warp
 
 
+@pytest.mark.parametrize("name", ["fmha_tc.cu", "fmha_sparse_tc.cu", "fmha_decode_tc.cu"])
+def test_a_timeout_outlasts_the_copies_in_flight(name):
+    """After a wait gave up, shared memory and TMEM are given back only once nothing that was issued can still land there."""
+    end = code(name).rsplit("if (*abort_flag) {", 1)[1]
+    assert end.index("outlast_async_work();") < end.index("tmem_dealloc(")
+
+
 def test_sparse_loader_leaves_before_the_wait():
     """A loader warp without a unit in the last chunk of a list may not wait for that chunk's buffer (the phase it waits for
     can be over by then).  That the condition is right for every group size and chunk is asserted when the file is compiled."""
