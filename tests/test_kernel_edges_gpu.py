@@ -23,9 +23,11 @@ def i32(v, device=None):
     (2, 300, 33, 32, 0, 0), (2, 300, 2000, 32, 3, 0),
     (3, 257, 9, 8, 0, 0), (5, 64, 5, 4, 0, 1), (1, 31, 9000, 16, 0, 0),
     (1, 32, 300, 16, 0, 0), (8, 32, 300, 16, 0, 0), (9, 32, 300, 16, 0, 0),    # either side of the row count of the rule
+    (2, 1100, 97, 32, 0, 0),
 ])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("kind", ["normal", "ties", "special"])
-def test_topk_edges(h, t, nvp, topk, fb, fe, kind):
+def test_topk_edges(h, t, nvp, topk, fb, fe, kind, dtype):
     import msa_for_sail as msa
     g = gen(h * 1000 + t + nvp)
     s = torch.randn(h, nvp + 3, t, generator=g)
@@ -37,6 +39,7 @@ def test_topk_edges(h, t, nvp, topk, fb, fe, kind):
         for i, v in enumerate((float("nan"), float("inf"), -float("inf"), 0.0, -0.0, 3.402823466e38, -3.402823466e38, 1e-45)):
             s[pick == i] = v
         s[:, :, ::5] = float("nan")
+    s = s.to(dtype)
     got = msa.sparse_topk_select(s.to(DEV), topk, num_valid_pages=nvp, force_begin_blocks=fb, force_end_blocks=fe)
     assert torch.equal(got.cpu(), orc.topk_select(s, topk, nvp, fb, fe))
 
