@@ -366,6 +366,20 @@ topk_row_kernel(const T* scores, int32_t* out, int num_heads, int max_k_tiles, i
   const int t = blockIdx.x % total_q, head = blockIdx.x / total_q;
   const T* base = scores + static_cast<size_t>(head) * max_k_tiles * total_q + t;
   uint32_t ord[NK], page[NK];
+  // All loads before any use, four at a time with one test.  (With the load beside its use the compiler only kept several on
+  // the way where it could take the scores as constant: 8 192 pages x 496 rows, topk 4: 25 us against 34.)
+  T score[NK];
+#pragma unroll
+  for (int i0 = 0; i0 < NK; i0 += 4) {
+    if (256 * (i0 + 4) <= nvp) {
+#pragma unroll
+      for (int i = i0; i < i0 + 4; ++i) score[i] = base[static_cast<size_t>(tid + 256 * i) * total_q];
+    } else {
+#pragma unroll
+      for (int i = i0; i < i0 + 4; ++i)
+        score[i] = tid + 256 * i < nvp ? base[static_cast<size_t>(tid + 256 * i) * total_q] : static_cast<T>(0.f);
+    }
+  }
 #pragma unroll
   for (int i = 0; i < NK; ++i) {
     const int pg = tid + 256 * i;
@@ -373,7 +387,7 @@ topk_row_kernel(const T* scores, int32_t* out, int num_heads, int max_k_tiles, i
     ord[i] = 0u;                                             // 0: not a candidate
     if (pg < nvp) {
       const bool forced = pg < force_begin || pg >= force_end_start;
-      ord[i] = forced ? kForcedOrd : ord_key(static_cast<float>(base[static_cast<size_t>(pg) * total_q]));
+      ord[i] = forced ? kForcedOrd : ord_key(static_cast<float>(score[i]));
     }
   }
   // level 1: this warp's TOPK best, winner r in lane r
