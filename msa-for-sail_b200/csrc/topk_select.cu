@@ -445,13 +445,18 @@ int launch(const T* scores, int32_t* out, int H, int K, int T_, int nvp, int fb,
   }
   const int fe_start = fe <= nvp ? nvp - fe : 0;
   const bool one_word = sizeof(T) == 2 && fb == 0 && fe == 0 && nvp <= 65535;      // bf16 scores, nothing forced
-  // Decode-sized: a CTA per row.  From 32 tokens on a thread-per-row kernel has its lanes filled, and past the rows that
-  // are resident at a few CTAs per SM it wins (1 024 rows x 256 pages: 7.5 us against 18.5; 32 rows x 1 024 pages, one
-  // CTA there: 10 us against 7.4).
-  if ((T_ < 32 || rows <= 256 || one_word) && rows <= 2048 && nvp <= 256 * 32) {
-    if (nvp <= 256 * 4)
+  // Decode-sized: a CTA per row, its pages in the registers of 256 threads (nk each).  From 32 tokens on a thread per row has
+  // its lanes filled.  That one's time grows with the pages alone as long as its CTAs are resident, the other's with rows x
+  // nk x topk from a few CTAs per SM on.  The line between them was fitted to both times at 1 456 sizes (32 to 2 048 rows, 33
+  // to 8 192 pages, topk 4 to 32, both types): 0.6 % above the faster one on average, at most 1.26 times it but for three
+  // sizes (1.7).  fp32, topk 16, CTA per row / thread per row: 32 rows x 1 024 pages 6.5 / 13.0 us, 384 x 2 048 17.6 / 21.9,
+  // 384 x 4 096 61 / 39, 1 024 x 256 18.1 / 6.6.
+  const int nk = nvp <= 256 * 4 ? 4 : (nvp <= 256 * 8 ? 8 : 32);
+  const bool cta_per_row = T_ < 32 || (static_cast<long long>(rows) + 150) * nk * TOPK <= 36LL * (nvp + 128);
+  if (cta_per_row && rows <= 2048 && nvp <= 256 * 32) {
+    if (nk == 4)
       launch_chained(topk_row_kernel<TOPK, 4, T>, static_cast<unsigned>(rows), 256, 0, stream, scores, out, H, K, T_, nvp, fb, fe_start);
-    else if (nvp <= 256 * 8)
+    else if (nk == 8)
       launch_chained(topk_row_kernel<TOPK, 8, T>, static_cast<unsigned>(rows), 256, 0, stream, scores, out, H, K, T_, nvp, fb, fe_start);
     else
       launch_chained(topk_row_kernel<TOPK, 32, T>, static_cast<unsigned>(rows), 256, 0, stream, scores, out, H, K, T_, nvp, fb, fe_start);

@@ -22,8 +22,10 @@ def i32(v, device=None):
     (1, 1000, 769, 16, 0, 0),
     (2, 300, 33, 32, 0, 0), (2, 300, 2000, 32, 3, 0),
     (3, 257, 9, 8, 0, 0), (5, 64, 5, 4, 0, 1), (1, 31, 9000, 16, 0, 0),
-    (1, 32, 300, 16, 0, 0), (8, 32, 300, 16, 0, 0), (9, 32, 300, 16, 0, 0),    # either side of the row count of the rule
-    (2, 1100, 97, 32, 0, 0),
+    # either side of the line between a CTA and a thread per row, by rows and by pages, and with 4, 8 and 32 pages a thread
+    (1, 32, 300, 16, 0, 0), (2, 32, 300, 16, 0, 0), (11, 33, 1024, 16, 0, 1), (11, 33, 1025, 16, 0, 0), (11, 33, 2048, 16, 0, 0),
+    (11, 33, 2049, 16, 0, 0), (11, 33, 8192, 16, 0, 0), (5, 40, 900, 8, 1, 0), (40, 50, 8000, 4, 0, 0), (40, 50, 700, 4, 0, 0),
+    (3, 33, 1100, 32, 0, 0), (3, 33, 900, 32, 0, 0), (2, 1100, 97, 32, 0, 0),
 ])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("kind", ["normal", "ties", "special"])
