@@ -2,7 +2,7 @@
 // index heads of one or a few query tokens, upstream sm80_fmha_fwd_mainloop.hpp:427-470 with output_o = false).
 //
 // HBM-bound: the K cache is read once (32 KB per bf16 page, 16 KB in e4m3), at up to 16 FLOP per byte.  A warp owns one
-// 128-key page at a time and streams it, 16 keys a stage, through its own 16 KB of shared memory (cp.async, whole
+// 128-key page at a time and streams it, 16 keys a stage, through shared memory of its own, 16 KB (cp.async, whole
 // 128-byte lines; nothing wider than a warp to synchronise).  The stages run on from page to page: up to 168 KB in
 // flight per SM without a gap.  Lane 4g + t works on pieces t, t + 4, ... (16 bytes each) of keys g and g + 8 of the
 // stage, and holds the same pieces of the rows of Q.
@@ -31,10 +31,19 @@ namespace score_stream {
 namespace {
 
 constexpr int BN = 128;
-constexpr int NWARPS = 12, NTHREADS = NWARPS * 32;
-constexpr int RING = 16 * 1024;                  // per warp
 constexpr int MAX_ITEMS = 4096;                  // work items numbered at a time
-constexpr int SMEM_BYTES = NWARPS * RING + (MAX_ITEMS + 1) * 4;
+// e4m3, four rows: 64 registers of Q and the conversions leave three warps per scheduler waiting; with four of them (and
+// rings of 8 KB, 128 KB in flight per SM) 32 sequences x 320 pages take 67 us instead of 75.
+// UNROLL: of the eight stages of a page.  Four rows are 256 multiply-adds a stage and lane: unrolled eight times that is more
+// code than the instruction caches hold (10 240 pages: bf16 71 -> 57 us, e4m3 67 -> 52 us with a loop; 2 pages: 8.6 -> 7.1 and
+// 9.2 -> 8.0 us).  One or two rows of bf16 are 1 to 2 % better with four stages; in e4m3 they are 5 % better with all eight.
+template <bool F8, int R>
+struct Cfg {
+  static constexpr int NWARPS = F8 && R == 4 ? 16 : 12, NTHREADS = NWARPS * 32;
+  static constexpr int RING = (F8 && R == 4 ? 8 : 16) * 1024;         // per warp
+  static constexpr int SMEM_BYTES = NWARPS * RING + (MAX_ITEMS + 1) * 4;
+  static constexpr int UNROLL = R == 4 ? 1 : (F8 ? 8 : 4);
+};
 
 // acc += a.lo * b.lo + a.hi * b.hi, operands packed f16x2 / bf16x2, fp32 accumulate
 template <bool F16>
@@ -60,15 +69,17 @@ __device__ __forceinline__ uint32_t e4m3x2_to_f16x2(uint32_t two_bytes) {
 
 // F8: e4m3 cache (q e4m3 or bf16, multiplied as f16); otherwise bf16 cache and bf16 q.  R: most rows of an item.
 template <bool F8, int R>
-__global__ void __launch_bounds__(NTHREADS, 1)
+__global__ void __launch_bounds__(Cfg<F8, R>::NTHREADS, 1)
 score_stream_kernel(const __grid_constant__ MsaFmhaParams p) {
+  using C = Cfg<F8, R>;
+  constexpr int NWARPS = C::NWARPS, NTHREADS = C::NTHREADS, RING = C::RING, UNROLL = C::UNROLL;
   constexpr bool MMA = R == 8;
   constexpr int QR = MMA ? 1 : R;                // rows of Q a lane holds (MMA: row g, the B fragments)
   constexpr int MR = MMA ? 2 : R;                // rows whose maximum a lane holds (MMA: rows 2t, 2t + 1)
   constexpr int PIECES = F8 ? 2 : 4;             // 16-byte pieces of a key per lane
   constexpr int STAGE = 2 * PIECES * 512;        // 16 keys: 2 KB in e4m3, 4 KB in bf16
   constexpr int STAGES = RING / STAGE;           // 8 or 4; a page is 8 stages
-  static_assert(8 % STAGES == 0, "the ring position is static in the loop over a page");
+  static_assert(8 % STAGES == 0, "a page starts at the first stage of the ring");
   extern __shared__ __align__(128) unsigned char s_score[];
   __shared__ int s_warp_sum[NWARPS];
   int* s_pref = reinterpret_cast<int*>(s_score + NWARPS * RING);     // [items + 1] pages before an item
@@ -220,7 +231,7 @@ score_stream_kernel(const __grid_constant__ MsaFmhaParams p) {
 #pragma unroll
         for (int m = 0; m < MR; ++m) mx[m] = -INFINITY;
         const bool all_visible = tile * BN + BN - 1 <= min_lim;
-#pragma unroll
+#pragma unroll UNROLL
         for (int u = 0; u < 8; ++u) {
           cp_async_wait<STAGES - 2>();
           __syncwarp();                                      // every lane's copies of this stage are in, its reads of the last one done
@@ -349,17 +360,21 @@ int score_stream_launch(const MsaFmhaParams& p, cudaStream_t stream) {
   const KernelFn kernels[8] = {score_stream_kernel<false, 1>, score_stream_kernel<false, 2>, score_stream_kernel<false, 4>,
                                score_stream_kernel<false, 8>, score_stream_kernel<true, 1>,  score_stream_kernel<true, 2>,
                                score_stream_kernel<true, 4>,  score_stream_kernel<true, 8>};
+  const int threads[8] = {Cfg<false, 1>::NTHREADS, Cfg<false, 2>::NTHREADS, Cfg<false, 4>::NTHREADS, Cfg<false, 8>::NTHREADS,
+                          Cfg<true, 1>::NTHREADS,  Cfg<true, 2>::NTHREADS,  Cfg<true, 4>::NTHREADS,  Cfg<true, 8>::NTHREADS};
+  const int smem[8] = {Cfg<false, 1>::SMEM_BYTES, Cfg<false, 2>::SMEM_BYTES, Cfg<false, 4>::SMEM_BYTES, Cfg<false, 8>::SMEM_BYTES,
+                       Cfg<true, 1>::SMEM_BYTES,  Cfg<true, 2>::SMEM_BYTES,  Cfg<true, 4>::SMEM_BYTES,  Cfg<true, 8>::SMEM_BYTES};
   const int rows = p.decode_rows;
   const int v = (p.kv_dtype == MSA_DT_E4M3 ? 4 : 0) + (rows <= 1 ? 0 : (rows <= 2 ? 1 : (rows <= 4 ? 2 : 3)));
   if (dev >= 16 || !attr_done[v][dev]) {
-    if (cudaFuncSetAttribute(kernels[v], cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
+    if (cudaFuncSetAttribute(kernels[v], cudaFuncAttributeMaxDynamicSharedMemorySize, smem[v]) != cudaSuccess)
       return MSA_ERR_LAUNCH;
     if (dev < 16) attr_done[v][dev] = true;
   }
   // one CTA per SM, fewer only where there cannot be a page for each
   const int64_t most_pages = static_cast<int64_t>(p.num_work) * std::max(1, p.max_k_tiles);
   const int grid = static_cast<int>(std::min<int64_t>(nsm, most_pages));
-  return launch_chained(kernels[v], grid, NTHREADS, SMEM_BYTES, stream, p) == cudaSuccess ? MSA_OK : MSA_ERR_LAUNCH;
+  return launch_chained(kernels[v], grid, threads[v], smem[v], stream, p) == cudaSuccess ? MSA_OK : MSA_ERR_LAUNCH;
 }
 
 }  // namespace msa
