@@ -88,9 +88,12 @@ constexpr bool loader_has_unit_agrees() {                  // with the dealing i
   return true;
 }
 static_assert(loader_has_unit_agrees(), "a loader leaves before the wait for a chunk exactly where it has no unit in it");
-// Chunks of 128 rows per work item: a list of one page in pieces of 32, of 16 where an SM gets fewer than 128 chunks in
-// all and the last round weighs more than the pages loaded twice (9 000 tokens x 16 heads x 8 pages: 193 us a pass
-// against 198; 8: 205.  65 536 chunks: 1 654 us with 16, 1 620 with 32; 524 288 chunks: 32, 64 and 128 within 1 %).
+// Chunks of 128 rows per work item: a list of one page in pieces of 32, of 16 where an SM of 148 gets fewer than 128 chunks
+// in all and the last round weighs more than the pages loaded twice.  77 batches of 2 500 to 18 900 chunks (one to seven
+// sequences, whole or with a prefix, both types): 16 is 3.6 % faster on average, 23 % at best, 6 % slower at worst; whole
+// prompts of one sequence with evenly spread selections have both, 7 % faster at 6 000 chunks and up to 10 % slower at 9 000 to
+// 16 000.  From 19 000 to 64 000 chunks 32 is 1 to 7 % faster, at 524 288 32, 64 and 128 are within 1 %.  (The host does not
+// know the lengths of the lists, and the workspace is sized by the same rule on every device: hence the fixed SM count.)
 inline int item_chunks(int64_t rows) { return rows < int64_t(148) * 128 * BM ? 16 : 32; }
 // Pairs (of 16 per 32 columns) whose exp2 runs on the FMA pipe.  At 2 x 32 768 tokens in bf16 a whole pass takes 10.6 ms
 // with none, 10.2 ms with two of 16 and 9.9 ms with six; in e4m3, whose conversions fill the ALU already, none is best

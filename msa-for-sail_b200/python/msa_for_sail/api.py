@@ -119,7 +119,9 @@ def _sparse_splits(items, kv_block_num, num_kv_splits, num_sms, two_per_sm):
     """Splits of the selected pages in token-major sparse attention, halved as often as pays.  A CTA takes its
     pages and about four page times more (dependent index loads, the first page's latency, the epilogue), the CTAs run in
     rounds of the slots there are (two e4m3 CTAs of at most 16 rows share an SM), and splits cost a merge, about four
-    page times.  24 tokens x 4 heads x 16 bf16 pages: 192 CTAs of 8 pages and the merge 36 us, 96 of 16 pages 26 us."""
+    page times.  Measured for 2 to 384 items of 4 to 32 pages in both types with every power of two up to 8: the count that
+    this gives is within 2 us (a step of the clock) of the best one at all 176 sizes; 24 tokens x 4 heads x 16 bf16 pages:
+    34 us uncut, 45 us in two, 59 us in eight, kernels alone on a cold L2."""
     # The most splits, which partials in a caller's workspace are sized for: enough CTAs for two rounds, or of an explicit
     # count what is left once halving it would leave an SM without a CTA.
     if num_kv_splits >= 1:
